@@ -31,7 +31,7 @@ def build(reference: str | None = None) -> None:
     """Build liboracle.so, and the reference pins when the reference tree is present."""
     subprocess.run(["make", "-s", "-C", str(HERE), "all"], check=True)
     ref = reference or os.environ.get("VFB_REFERENCE_DIR", "/root/reference")
-    if Path(ref).is_dir():
+    if (Path(ref) / "src" / "lbm" / "ChimeraTransformation.h").is_file():    # an empty mount point is no tree
         subprocess.run(["make", "-s", "-C", str(HERE), "ref", f"REF={ref}"], check=True)
 
 

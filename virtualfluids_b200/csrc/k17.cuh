@@ -14,6 +14,8 @@
 //    4th, 5th and 6th order cumulants are multiplied by zero (4th) or relaxed to exactly zero
 //    (5th, 6th), so they are not computed here; for finite inputs this changes no value.
 #pragma once
+#include <cmath>
+
 #include "lattice.cuh"
 
 namespace vfb {
@@ -31,6 +33,11 @@ struct K17Rates {
     T m3w;                      // -3 * omega
     T c3a;                      // 3 * (1 + 1/2 * (-omega))
     T omOxyz, omOP, omOM;       // 1 - Oxyz, 1 - OxyyPxzz, 1 - OxyyMxzz
+    // folded constants of the FMA form (k17_collide_fast)
+    T omo;                      // 1 - omega
+    T mc3h;                     // -3 (1 - omega / 2)
+    T hP, hM, cD;               // 1/2 (1 - OxyyPxzz) qP, 1/2 (1 - OxyyMxzz) qM, (1 - Oxyz) qD
+    T kA, kB;                   // neg_iwm 2/3 factorA, neg_iwm 1/3 factorB (-3 omega)
 };
 
 // host computation of the omega-only rates, expression for expression as the reference
@@ -56,6 +63,13 @@ inline K17Rates<T> make_k17_rates(T omega, T qP, T qM, T qD)
     r.omOxyz = T(1) - r.Oxyz;
     r.omOP = T(1) - r.OxyyPxzz;
     r.omOM = T(1) - r.OxyyMxzz;
+    r.omo = T(1) - w;
+    r.mc3h = T(-3) * (T(1) - T(0.5) * w);
+    r.hP = T(0.5) * r.omOP * qP;
+    r.hM = T(0.5) * r.omOM * qM;
+    r.cD = r.omOxyz * qD;
+    r.kA = r.neg_iwm * (T(2) / T(3)) * r.factorA;
+    r.kB = r.neg_iwm * (T(1) / T(3)) * r.factorB * r.m3w;
     return r;
 }
 
@@ -396,79 +410,55 @@ __host__ __device__ __forceinline__ void k17_collide(T *f, const K17Rates<T> &r,
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same collision, rearranged for fewer floating-point instructions (the FMA variant).
+// The same collision, rearranged for fewer floating-point instructions (the FMA variant): 495
+// operations and eight reciprocals per node. Mathematically identical to k17_collide, rounded
+// differently:
+//  * the populations are summed to raw moments (three additions per line, no velocity), which hold
+//    density and momentum; only the moments up to third order are shifted to the velocity, with
+//    the shifts of lower moments shared (j' = j - rho u, p = m_ab - u_b j_a). A transform line by
+//    line, velocity in every line, took 100 operations more;
+//  * a limited rate O + (1 - O) |m| / (|m| + q) leaves m (1 - O) q / (|m| + q) of its moment;
+//  * with M = m + 1/3 for the second moments, c_s^2 terms and products of the post-collision
+//    moments group to M m (e.g. 3 (xx y + 2 ..) + y = 3 ((xx + 1/3) y + ..));
+//  * a backward line forms S = c + w v^2 + 2 b v and D = b + w v (w = a + K, the K offset of the
+//    well-conditioned populations): its results are (S - D) / 2, a - S, (S + D) / 2.
+// The error against 64 bits is that of the line-by-line form or less (FP32, 20000 random states per
+// omega and velocity scale: 1.5e-7 .. 1.9e-7 of the populations against 2.0e-7 .. 2.5e-7).
 //
-// Mathematically identical to k17_collide, rounded differently:
-//  * the well-conditioned chimera transforms are used in their K-offset form,
-//    b' = m1 - v (m0 + K), c' = m2 - 2 v m1 + v^2 (m0 + K) (forward) and the matching backward
-//    form -- the reference's forwardChimeraWithK / backwardChimeraWithK
-//    (src/lbm/ChimeraTransformation.h:124-150) -- since (x K^-1 + 1) K = x + K;
-//  * density and momenta share the 13 pair sums and differences f_d +- f_inv(d);
-//  * the eight reciprocals of a node (1/rho and the seven quartic-limiter denominators) come from
-//    one division (product of the denominators, then back-substitution);
-//  * omega-only products are folded into single constants.
+// T is an arithmetic type whose operations each round on their own (Rn below, or the packed f2), so
+// the compiler contracts nothing and every kernel computes the same bits from the same
+// populations: a box, a pool domain, a list level, one node per thread or two.
 // ---------------------------------------------------------------------------------------------
-template <class T>
-struct K17FastConst {
-    T omega;
-    T OxyyPxzz, OxyyMxzz, Oxyz;
-    T kA;       // -(1/omega - 1/2) * 2/3 * factorA
-    T kB;       // -(1/omega - 1/2) * 1/3 * factorB
-    T qP, qM, qD;
-};
 
-template <class T>
-__host__ __device__ inline K17FastConst<T> make_k17_fast_const(const K17Rates<T> &r)
-{
-    K17FastConst<T> c;
-    c.omega = r.omega;
-    c.OxyyPxzz = r.OxyyPxzz;
-    c.OxyyMxzz = r.OxyyMxzz;
-    c.Oxyz = r.Oxyz;
-    c.kA = r.neg_iwm * (T(2) / T(3)) * r.factorA;
-    c.kB = r.neg_iwm * (T(1) / T(3)) * r.factorB;
-    c.qP = r.qP;
-    c.qM = r.qM;
-    c.qD = r.qD;
-    return c;
-}
+// one value with operations that are never contracted
+template <class B>
+struct Rn {
+    B v;
+    Rn() = default;
+    __host__ __device__ __forceinline__ Rn(B a) : v(a) {}
+};
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float rn_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float rn_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rn_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double rn_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double rn_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+#else
+template <class B> inline B rn_add(B a, B b) { return a + b; }
+template <class B> inline B rn_mul(B a, B b) { return a * b; }
+template <class B> inline B rn_fma(B a, B b, B c) { return std::fma(a, b, c); }
+#endif
+template <class B> __host__ __device__ __forceinline__ Rn<B> operator+(Rn<B> a, Rn<B> b) { return rn_add(a.v, b.v); }
+template <class B> __host__ __device__ __forceinline__ Rn<B> operator-(Rn<B> a, Rn<B> b) { return rn_add(a.v, -b.v); }
+template <class B> __host__ __device__ __forceinline__ Rn<B> operator*(Rn<B> a, Rn<B> b) { return rn_mul(a.v, b.v); }
+template <class B> __host__ __device__ __forceinline__ Rn<B> operator-(Rn<B> a) { return Rn<B>(-a.v); }
+template <class B> __host__ __device__ __forceinline__ Rn<B> fma(Rn<B> a, Rn<B> b, Rn<B> c) { return rn_fma(a.v, b.v, c.v); }
 
 namespace k17detail {
-// forward transform along one line with offset K (K = 0: the plain central-moment transform);
-// K is a constant of the unrolled loops, so the K = 0 lines carry no offset addition
-template <class T>
-__host__ __device__ __forceinline__ void fwdK(T &a, T &b, T &c, T v, T v2, T twov, T K)
-{
-    const T apc = a + c;
-    const T m1 = c - a;
-    const T m0 = apc + b;
-    const T w = K == T(0) ? m0 : m0 + K;
-    a = m0;
-    b = fma(-v, w, m1);
-    c = fma(v2, w, fma(-twov, m1, apc));
-}
-// backward transform with offset K: a' = ((c - b) + w (v^2 - v))/2 + b v,
-// b' = (a - c) - 2 b v - w v^2, c' = ((c + b) + w (v^2 + v))/2 + b v, w = a + K
-template <class T>
-__host__ __device__ __forceinline__ void bwdK(T &a, T &b, T &c, T v, T v2mv, T v2pv, T twov, T v2, T K)
-{
-    (void)twov;
-    const T w = K == T(0) ? a : a + K;
-    const T bv = b * v;
-    const T r0 = fma(T(0.5), fma(w, v2mv, c - b), bv);
-    const T r1 = fma(-v2, w, fma(T(-2), bv, a - c));
-    c = fma(T(0.5), fma(w, v2pv, c + b), bv);
-    a = r0;
-    b = r1;
-}
 // 1/x: IEEE division in double; the fast approximate division in float
-template <class T>
-__host__ __device__ __forceinline__ T fast_rcp(T x)
-{
-    return T(1) / x;
-}
-template <>
-__host__ __device__ __forceinline__ float fast_rcp<float>(float x)
+__host__ __device__ __forceinline__ double fast_rcp(double x) { return 1.0 / x; }
+__host__ __device__ __forceinline__ float fast_rcp(float x)
 {
 #ifdef __CUDA_ARCH__
     return __fdividef(1.0f, x);
@@ -485,13 +475,8 @@ __host__ __device__ __forceinline__ float fast_rcp<float>(float x)
 // reciprocal flushes subnormals (rcp.rn.ftz): rho is near 1, so the bits are those of the IEEE
 // reciprocal, and the form without flushing carries a slow path whose call raised the 16-bit
 // pool kernel from 128 to 172 registers.
-template <class T>
-__host__ __device__ __forceinline__ T rho_rcp(T x)
-{
-    return T(1) / x;
-}
-template <>
-__host__ __device__ __forceinline__ float rho_rcp<float>(float x)
+__host__ __device__ __forceinline__ double rho_rcp(double x) { return 1.0 / x; }
+__host__ __device__ __forceinline__ float rho_rcp(float x)
 {
 #ifdef __CUDA_ARCH__
     float y;
@@ -501,66 +486,69 @@ __host__ __device__ __forceinline__ float rho_rcp<float>(float x)
     return 1.0f / x;
 #endif
 }
-
-// the seven limiter reciprocals: in double one division and back-substitution through the
-// running products (the denominators are >= the limiters, so the product stays far above the
-// double range limit); in float seven fast divisions (a float product could underflow)
-template <class T>
-__host__ __device__ __forceinline__ void limiter_inverses(const T (&d)[7], T (&iv)[7])
+template <class B>
+__host__ __device__ __forceinline__ Rn<B> rho_rcp(Rn<B> x)
 {
-    const T p1 = d[0] * d[1], p2 = p1 * d[2], p3 = p2 * d[3], p4 = p3 * d[4], p5 = p4 * d[5], p6 = p5 * d[6];
-    T rr = T(1) / p6;
-    iv[6] = rr * p5;
-    rr *= d[6];
-    iv[5] = rr * p4;
-    rr *= d[5];
-    iv[4] = rr * p3;
-    rr *= d[4];
-    iv[3] = rr * p2;
-    rr *= d[3];
-    iv[2] = rr * p1;
-    rr *= d[2];
-    iv[1] = rr * d[0];
-    iv[0] = rr * d[1];
+    return rho_rcp(x.v);
 }
-template <>
-__host__ __device__ __forceinline__ void limiter_inverses<float>(const float (&d)[7], float (&iv)[7])
+
+// 1 / (|m_i| + q_i) of the seven limited moments: in double one division and back-substitution
+// through the running products (the denominators are >= the limiters, so the product stays far
+// above the double range limit); in float seven fast divisions (a float product could underflow)
+__host__ __device__ __forceinline__ void limiter_inverses(const Rn<double> (&m)[7], const double (&q)[7],
+                                                          Rn<double> (&iv)[7])
+{
+    Rn<double> d[7], p[7];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        d[i] = Rn<double>(fabs(m[i].v)) + Rn<double>(q[i]);
+        p[i] = i == 0 ? d[0] : p[i - 1] * d[i];
+    }
+    Rn<double> rr = fast_rcp(p[6].v);
+#pragma unroll
+    for (int i = 6; i > 0; --i) {
+        iv[i] = rr * p[i - 1];
+        rr = rr * d[i];
+    }
+    iv[0] = rr;
+}
+__host__ __device__ __forceinline__ void limiter_inverses(const Rn<float> (&m)[7], const float (&q)[7],
+                                                          Rn<float> (&iv)[7])
 {
 #pragma unroll
     for (int i = 0; i < 7; ++i)
-        iv[i] = fast_rcp<float>(d[i]);
+        iv[i] = fast_rcp(rn_add(fabsf(m[i].v), q[i]));
+}
+
+// raw moments 0, 1, 2 of one line
+template <class T>
+__host__ __device__ __forceinline__ void raw_line(T &a, T &b, T &c)
+{
+    const T p = c + a;
+    const T q = c - a;
+    a = p + b;
+    b = q;
+    c = p;
+}
+// central moments a, b, c of one line back to its populations; w = a + K
+template <class T>
+__host__ __device__ __forceinline__ void back_line(T &a, T &b, T &c, T v, T v2, T twov, T w, T half, T mhalf)
+{
+    const T S = fma(twov, b, fma(v2, w, c));
+    const T D = fma(v, w, b);
+    const T Sh = S * half;
+    b = a - S;
+    a = fma(mhalf, D, Sh);
+    c = fma(half, D, Sh);
 }
 } // namespace k17detail
 
-template <class T>
-__host__ __device__ __forceinline__ void k17_collide_fast(T *f, const K17FastConst<T> &r, T fx, T fy, T fz, T &drho_out,
-                                                 T &vx_out, T &vy_out, T &vz_out)
+// T: the arithmetic type, B: its base type (constants and rates)
+template <class T, class B>
+__host__ __device__ __forceinline__ void k17_collide_fast(T *f, const K17Rates<B> &r, B fx, B fy, B fz, T &drho_out,
+                                                          T &vx_out, T &vy_out, T &vz_out)
 {
     using namespace k17detail;
-    // pair sums / differences, canonical direction first
-    const T s1 = f[1] + f[2], t1 = f[1] - f[2];       // P00
-    const T s3 = f[3] + f[4], t3 = f[3] - f[4];       // 0P0
-    const T s5 = f[5] + f[6], t5 = f[5] - f[6];       // 00P
-    const T s7 = f[7] + f[8], t7 = f[7] - f[8];       // PP0
-    const T s9 = f[9] + f[10], t9 = f[9] - f[10];     // PM0
-    const T s11 = f[11] + f[12], t11 = f[11] - f[12]; // P0P
-    const T s13 = f[13] + f[14], t13 = f[13] - f[14]; // P0M
-    const T s15 = f[15] + f[16], t15 = f[15] - f[16]; // 0PP
-    const T s17 = f[17] + f[18], t17 = f[17] - f[18]; // 0PM
-    const T s19 = f[19] + f[26], t19 = f[19] - f[26]; // PPP
-    const T s21 = f[21] + f[24], t21 = f[21] - f[24]; // PMP
-    const T s23 = f[23] + f[22], t23 = f[23] - f[22]; // PPM
-    const T s25 = f[25] + f[20], t25 = f[25] - f[20]; // PMM
-    const T drho = ((((s19 + s21) + (s23 + s25)) + ((s7 + s9) + (s11 + s13))) + ((s15 + s17) + (s1 + s3))) + (s5 + f[0]);
-    const T jx = (((t19 + t21) + (t23 + t25)) + ((t7 + t9) + (t11 + t13))) + t1;
-    const T jy = (((t19 - t21) + (t23 - t25)) + ((t7 - t9) + (t15 + t17))) + t3;
-    const T jz = (((t19 + t21) - (t23 + t25)) + ((t11 - t13) + (t15 - t17))) + t5;
-
-    const T oneOverRho = rho_rcp(drho + T(1));
-    const T vx = fma(jx, oneOverRho, fx), vy = fma(jy, oneOverRho, fy), vz = fma(jz, oneOverRho, fz);
-    const T vx2 = vx * vx, vy2 = vy * vy, vz2 = vz * vz;
-    const T twovx = T(2) * vx, twovy = T(2) * vy, twovz = T(2) * vz;
-
     T m[27];
 #pragma unroll
     for (int d = 0; d < 27; ++d)
@@ -570,133 +558,137 @@ __host__ __device__ __forceinline__ void k17_collide_fast(T *f, const K17FastCon
     for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int b = 0; b < 3; ++b)
-            fwdK(M(a, b, 0), M(a, b, 1), M(a, b, 2), vz, vz2, twovz, k_z<T>(a, b));
+            raw_line(M(a, b, 0), M(a, b, 1), M(a, b, 2));
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-            fwdK(M(a, 0, c), M(a, 1, c), M(a, 2, c), vy, vy2, twovy, c == 1 ? T(0) : k_y<T>(a, c));
+            raw_line(M(a, 0, c), M(a, 1, c), M(a, 2, c));
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            raw_line(M(0, b, c), M(1, b, c), M(2, b, c));
+
+    const T half = T(B(0.5)), mhalf = T(B(-0.5)), third = T(B(1) / B(3));
+    const T drho = M(0, 0, 0), jx = M(1, 0, 0), jy = M(0, 1, 0), jz = M(0, 0, 1);
+    const T rho = drho + T(B(1));
+    const T ir = rho_rcp(rho);
+    const T vx = fma(jx, ir, T(fx)), vy = fma(jy, ir, T(fy)), vz = fma(jz, ir, T(fz));
+    const T mvx = -vx, mvy = -vy, mvz = -vz;
+    // central moments up to third order (second ones without c_s^2: xx = sum (c_x - u_x)^2 f - 1/3)
+    const T tx = fma(mvx, rho, jx), ty = fma(mvy, rho, jy), tz = fma(mvz, rho, jz);
+    const T m200 = M(2, 0, 0), m020 = M(0, 2, 0), m002 = M(0, 0, 2);
+    const T xx0 = fma(mvx, jx + tx, m200), yy0 = fma(mvy, jy + ty, m020), zz0 = fma(mvz, jz + tz, m002);
+    const T pxy = fma(mvy, jx, M(1, 1, 0)), pxz = fma(mvz, jx, M(1, 0, 1)), pyz = fma(mvz, jy, M(0, 1, 1));
+    const T qxy = fma(mvx, jy, M(1, 1, 0)), qxz = fma(mvx, jz, M(1, 0, 1)), qyz = fma(mvy, jz, M(0, 1, 1));
+    const T xy0 = fma(mvx, ty, pxy), xz0 = fma(mvx, tz, pxz), yz0 = fma(mvy, tz, pyz);
+    const T a200 = m200 + third, a020 = m020 + third, a002 = m002 + third;
+    const T k210 = fma(mvx, pxy + xy0, fma(mvy, a200, M(2, 1, 0)));
+    const T k120 = fma(mvy, qxy + xy0, fma(mvx, a020, M(1, 2, 0)));
+    const T k201 = fma(mvx, pxz + xz0, fma(mvz, a200, M(2, 0, 1)));
+    const T k102 = fma(mvz, qxz + xz0, fma(mvx, a002, M(1, 0, 2)));
+    const T k021 = fma(mvy, pyz + yz0, fma(mvz, a020, M(0, 2, 1)));
+    const T k012 = fma(mvz, qyz + yz0, fma(mvy, a002, M(0, 1, 2)));
+    const T k111 = fma(mvx, yz0, fma(mvy, pxz, fma(mvz, M(1, 1, 0), M(1, 1, 1))));
+
+    // velocity gradients times rho and the second order relaxation (K17...h:347-387)
+    const T vx2 = vx * vx, vy2 = vy * vy, vz2 = vz * vz;
+    const T dy0 = xx0 - yy0, dz0 = xx0 - zz0;
+    const T gx = fma(T(r.mhw), dy0 + dz0, half * (drho - ((xx0 + yy0) + zz0)));
+    const T gy = fma(T(r.w32), dy0, gx), gz = fma(T(r.w32), dz0, gx);
+    const T ax = vx2 * gx, ay = vy2 * gy, az = vz2 * gz;
+    const T trace = fma(T(B(-1.5)), (ax + ay) + az, drho);
+    const T dy = fma(T(r.mc3h), ax - ay, T(r.omo) * dy0), dz = fma(T(r.mc3h), ax - az, T(r.omo) * dz0);
+    const T xy = T(r.omo) * xy0, xz = T(r.omo) * xz0, yz = T(r.omo) * yz0;
+
+    // third order with the quartic limiter (K17...h:397-433)
+    const T lm[7] = { k111, k210 + k012, k201 + k021, k120 + k102, k210 - k012, k201 - k021, k120 - k102 };
+    const B lq[7] = { r.qD, r.qP, r.qP, r.qP, r.qM, r.qM, r.qM };
+    T li[7];
+    limiter_inverses(lm, lq, li);
+    const T c111 = (lm[0] * T(r.cD)) * li[0];
+    const T px = (lm[1] * T(r.hP)) * li[1], mx = (lm[4] * T(r.hM)) * li[4];
+    const T py = (lm[2] * T(r.hP)) * li[2], my = (lm[5] * T(r.hM)) * li[5];
+    const T pz = (lm[3] * T(r.hP)) * li[3], mz = (lm[6] * T(r.hM)) * li[6];
+    const T c210 = px + mx, c012 = px - mx, c201 = py + my, c021 = py - my, c120 = pz + mz, c102 = pz - mz;
+
+    // central moments from the post-collision cumulants (K17...h:443-505)
+    const T xx = ((dy + dz) + trace) * third, yy = xx - dy, zz = xx - dz;
+    const T X = xx + third, Y = yy + third, Z = zz + third;
+    const T xy2 = xy + xy, xz2 = xz + xz, yz2 = yz + yz;
+    const T xy4 = xy2 + xy2, xz4 = xz2 + xz2, yz4 = yz2 + yz2;
+    const T sxy = xy2 * xy, sxz = xz2 * xz, syz = yz2 * yz;
+    const T u = xy2 * xz;
+    const T c211 = fma(ir, fma(X, yz, u), T(r.kB) * yz0);
+    const T c121 = fma(ir, fma(Y, xz, xy2 * yz), T(r.kB) * xz0);
+    const T c112 = fma(ir, fma(Z, xy, xz2 * yz), T(r.kB) * xy0);
+    const T y3 = yy * third, z3 = zz * third, d9 = drho * T(B(1) / B(9));
+    const T z3d = z3 - d9;
+    const T c220 = fma(ir, fma(xx, Y, (y3 - d9) + sxy), T(r.kA) * (gx + gy));
+    const T c202 = fma(ir, fma(xx, Z, z3d + sxz), T(r.kA) * (gx + gz));
+    const T c022 = fma(ir, fma(yy, Z, z3d + syz), T(r.kA) * (gy + gz));
+    const T c122 = ir * fma(Z, c120, fma(Y, c102, fma(yz4, c111, fma(xz2, c021, xy2 * c012))));
+    const T c212 = ir * fma(Z, c210, fma(X, c012, fma(xz4, c111, fma(yz2, c201, xy2 * c102))));
+    const T c221 = ir * fma(X, c021, fma(Y, c201, fma(xy4, c111, fma(xz2, c120, yz2 * c210))));
+    const T g3 = fma(xx, Y * Z, third * fma(yy, Z, z3));
+    const T e2 = fma(T(B(2)), fma(u, yz4, fma(sxz, Y, fma(syz, X, fma(sxy, Z, g3)))),
+                     T(B(1) / B(27)) * fma(drho, drho, -drho));
+    const T c111t = c111 + c111;
+    const T e0 = fma(Z, c220, fma(c111t, c111t, T(B(1) / B(9)) * trace));
+    const T e1 = fma(yz4, c211, fma(xz4, c121, fma(xy4, c112, fma(X, c022, fma(Y, c202, e0)))));
+    const T e3 = fma(T(B(2)), fma(c120, c102, fma(c210, c012, c201 * c021)), e1);
+    const T c222 = ir * fma(-ir, e2, e3);
+
+    // first moments change sign (K17...h:512-514)
+    M(1, 0, 0) = -tx;
+    M(0, 1, 0) = -ty;
+    M(0, 0, 1) = -tz;
+    M(2, 0, 0) = xx;
+    M(0, 2, 0) = yy;
+    M(0, 0, 2) = zz;
+    M(1, 1, 0) = xy;
+    M(1, 0, 1) = xz;
+    M(0, 1, 1) = yz;
+    M(1, 1, 1) = c111;
+    M(2, 1, 0) = c210;
+    M(0, 1, 2) = c012;
+    M(2, 0, 1) = c201;
+    M(0, 2, 1) = c021;
+    M(1, 2, 0) = c120;
+    M(1, 0, 2) = c102;
+    M(2, 1, 1) = c211;
+    M(1, 2, 1) = c121;
+    M(1, 1, 2) = c112;
+    M(2, 2, 0) = c220;
+    M(2, 0, 2) = c202;
+    M(0, 2, 2) = c022;
+    M(1, 2, 2) = c122;
+    M(2, 1, 2) = c212;
+    M(2, 2, 1) = c221;
+    M(2, 2, 2) = c222;
+    const T twovx = vx + vx, twovy = vy + vy, twovz = vz + vz;
 #pragma unroll
     for (int b = 0; b < 3; ++b)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const T K = (b == 0 && c == 0) ? T(1) : ((b == 2 || c == 2) && b != 1 && c != 1) ? T(1) / T(3) : T(0);
-            fwdK(M(0, b, c), M(1, b, c), M(2, b, c), vx, vx2, twovx, K);
-        }
-    // K17...h:222 transforms the (2,2) x-line with K^-1 = 3 but K = 1/9: the offset is 1/K^-1 = 1/3
-    // and the two higher moments come out scaled by K^-1 K = 1/3
-    M(1, 2, 2) *= T(1) / T(3);
-    M(2, 2, 2) *= T(1) / T(3);
-
-    const T c13 = T(1) / T(3), c19 = T(1) / T(9), c23 = T(2) / T(3), c127 = T(1) / T(27), h = T(0.5);
-    const T omega = r.omega;
-
-    T mxxPyyPzz = M(2, 0, 0) + M(0, 2, 0) + M(0, 0, 2);
-    T mxxMyy = M(2, 0, 0) - M(0, 2, 0);
-    T mxxMzz = M(2, 0, 0) - M(0, 0, 2);
-    T mxxyPyzz = M(2, 1, 0) + M(0, 1, 2);
-    T mxxyMyzz = M(2, 1, 0) - M(0, 1, 2);
-    T mxxzPyyz = M(2, 0, 1) + M(0, 2, 1);
-    T mxxzMyyz = M(2, 0, 1) - M(0, 2, 1);
-    T mxyyPxzz = M(1, 2, 0) + M(1, 0, 2);
-    T mxyyMxzz = M(1, 2, 0) - M(1, 0, 2);
-
-    const T m3omega = -T(3) * omega;
-    const T Dxy = m3omega * M(1, 1, 0);
-    const T Dxz = m3omega * M(1, 0, 1);
-    const T Dyz = m3omega * M(0, 1, 1);
-    const T dxux = fma(-h * omega, mxxMyy + mxxMzz, h * (M(0, 0, 0) - mxxPyyPzz));
-    const T o32 = omega * T(1.5);
-    const T dyuy = fma(o32, mxxMyy, dxux);
-    const T dzuz = fma(o32, mxxMzz, dxux);
-
-    const T c3h = T(3) * (T(1) - h * omega);
-    mxxPyyPzz += (M(0, 0, 0) - mxxPyyPzz) - T(1.5) * (vx2 * dxux + vy2 * dyuy + vz2 * dzuz);
-    mxxMyy = fma(-omega, mxxMyy, mxxMyy) - c3h * (vx2 * dxux - vy2 * dyuy);
-    mxxMzz = fma(-omega, mxxMzz, mxxMzz) - c3h * (vx2 * dxux - vz2 * dzuz);
-    const T omo = T(1) - omega;
-    M(0, 1, 1) *= omo;
-    M(1, 0, 1) *= omo;
-    M(1, 1, 0) *= omo;
-
-    // quartic limiters: seven reciprocals from one division
-    const T a0 = fabs(M(1, 1, 1)), a1 = fabs(mxxyPyzz), a2 = fabs(mxxyMyzz), a3 = fabs(mxxzPyyz);
-    const T a4 = fabs(mxxzMyyz), a5 = fabs(mxyyPxzz), a6 = fabs(mxyyMxzz);
-    const T dd[7] = { a0 + r.qD, a1 + r.qP, a2 + r.qM, a3 + r.qP, a4 + r.qM, a5 + r.qP, a6 + r.qM };
-    T iv[7];
-    limiter_inverses<T>(dd, iv);
-    const T i0 = iv[0], i1 = iv[1], i2 = iv[2], i3 = iv[3], i4 = iv[4], i5 = iv[5], i6 = iv[6];
-    // m += (O + (1-O) |m|/(|m|+q)) (-m)
-    M(1, 1, 1) -= fma(T(1) - r.Oxyz, a0 * i0, r.Oxyz) * M(1, 1, 1);
-    mxxyPyzz -= fma(T(1) - r.OxyyPxzz, a1 * i1, r.OxyyPxzz) * mxxyPyzz;
-    mxxyMyzz -= fma(T(1) - r.OxyyMxzz, a2 * i2, r.OxyyMxzz) * mxxyMyzz;
-    mxxzPyyz -= fma(T(1) - r.OxyyPxzz, a3 * i3, r.OxyyPxzz) * mxxzPyyz;
-    mxxzMyyz -= fma(T(1) - r.OxyyMxzz, a4 * i4, r.OxyyMxzz) * mxxzMyyz;
-    mxyyPxzz -= fma(T(1) - r.OxyyPxzz, a5 * i5, r.OxyyPxzz) * mxyyPxzz;
-    mxyyMxzz -= fma(T(1) - r.OxyyMxzz, a6 * i6, r.OxyyMxzz) * mxyyMxzz;
-
-    M(2, 0, 0) = c13 * (mxxMyy + mxxMzz + mxxPyyPzz);
-    M(0, 2, 0) = c13 * (-T(2) * mxxMyy + mxxMzz + mxxPyyPzz);
-    M(0, 0, 2) = c13 * (mxxMyy - T(2) * mxxMzz + mxxPyyPzz);
-    M(2, 1, 0) = (mxxyMyzz + mxxyPyzz) * h;
-    M(0, 1, 2) = (mxxyPyzz - mxxyMyzz) * h;
-    M(2, 0, 1) = (mxxzMyyz + mxxzPyyz) * h;
-    M(0, 2, 1) = (mxxzPyyz - mxxzMyyz) * h;
-    M(1, 2, 0) = (mxyyMxzz + mxyyPxzz) * h;
-    M(1, 0, 2) = (mxyyPxzz - mxyyMxzz) * h;
-
-    const T cm022 = r.kA * (dyuy + dzuz);
-    const T cm202 = r.kA * (dxux + dzuz);
-    const T cm220 = r.kA * (dyuy + dxux);
-    const T cm112 = r.kB * Dxy;
-    const T cm121 = r.kB * Dxz;
-    const T cm211 = r.kB * Dyz;
-
-    const T c13r = c13 * oneOverRho;
-    const T drr = drho * oneOverRho;
-    M(2, 1, 1) = fma(c13r, (T(3) * M(2, 0, 0) + T(1)) * M(0, 1, 1) + T(6) * M(1, 1, 0) * M(1, 0, 1), cm211);
-    M(1, 2, 1) = fma(c13r, (T(3) * M(0, 2, 0) + T(1)) * M(1, 0, 1) + T(6) * M(1, 1, 0) * M(0, 1, 1), cm121);
-    M(1, 1, 2) = fma(c13r, (T(3) * M(0, 0, 2) + T(1)) * M(1, 1, 0) + T(6) * M(1, 0, 1) * M(0, 1, 1), cm112);
-    M(2, 2, 0) = cm220 + ((T(9) * (M(2, 0, 0) * M(0, 2, 0) + T(2) * M(1, 1, 0) * M(1, 1, 0)) + T(3) * (M(2, 0, 0) + M(0, 2, 0))) * oneOverRho - drr) * c19;
-    M(2, 0, 2) = cm202 + ((T(9) * (M(2, 0, 0) * M(0, 0, 2) + T(2) * M(1, 0, 1) * M(1, 0, 1)) + T(3) * (M(2, 0, 0) + M(0, 0, 2))) * oneOverRho - drr) * c19;
-    M(0, 2, 2) = cm022 + ((T(9) * (M(0, 0, 2) * M(0, 2, 0) + T(2) * M(0, 1, 1) * M(0, 1, 1)) + T(3) * (M(0, 0, 2) + M(0, 2, 0))) * oneOverRho - drr) * c19;
-    M(1, 2, 2) = c13r * (T(3) * (M(0, 0, 2) * M(1, 2, 0) + M(0, 2, 0) * M(1, 0, 2) + T(4) * M(0, 1, 1) * M(1, 1, 1) + T(2) * (M(1, 0, 1) * M(0, 2, 1) + M(1, 1, 0) * M(0, 1, 2))) + (M(1, 2, 0) + M(1, 0, 2)));
-    M(2, 1, 2) = c13r * (T(3) * (M(0, 0, 2) * M(2, 1, 0) + M(2, 0, 0) * M(0, 1, 2) + T(4) * M(1, 0, 1) * M(1, 1, 1) + T(2) * (M(0, 1, 1) * M(2, 0, 1) + M(1, 1, 0) * M(1, 0, 2))) + (M(2, 1, 0) + M(0, 1, 2)));
-    M(2, 2, 1) = c13r * (T(3) * (M(2, 0, 0) * M(0, 2, 1) + M(0, 2, 0) * M(2, 0, 1) + T(4) * M(1, 1, 0) * M(1, 1, 1) + T(2) * (M(1, 0, 1) * M(1, 2, 0) + M(0, 1, 1) * M(2, 1, 0))) + (M(0, 2, 1) + M(2, 0, 1)));
-    const T r2 = oneOverRho * oneOverRho;
-    M(2, 2, 2) = -((-T(4) * M(1, 1, 1) * M(1, 1, 1) - (M(2, 0, 0) * M(0, 2, 2) + M(0, 2, 0) * M(2, 0, 2) + M(0, 0, 2) * M(2, 2, 0))
-                    - T(4) * (M(0, 1, 1) * M(2, 1, 1) + M(1, 0, 1) * M(1, 2, 1) + M(1, 1, 0) * M(1, 1, 2))
-                    - T(2) * (M(1, 2, 0) * M(1, 0, 2) + M(2, 1, 0) * M(0, 1, 2) + M(2, 0, 1) * M(0, 2, 1))) * oneOverRho
-                   + (T(4) * (M(1, 0, 1) * M(1, 0, 1) * M(0, 2, 0) + M(0, 1, 1) * M(0, 1, 1) * M(2, 0, 0) + M(1, 1, 0) * M(1, 1, 0) * M(0, 0, 2))
-                      + T(2) * (M(2, 0, 0) * M(0, 2, 0) * M(0, 0, 2)) + T(16) * M(1, 1, 0) * M(1, 0, 1) * M(0, 1, 1)) * r2
-                   - (c13 * (M(0, 2, 2) + M(2, 0, 2) + M(2, 2, 0)) + c19 * (M(2, 0, 0) + M(0, 2, 0) + M(0, 0, 2))) * oneOverRho
-                   + (T(2) * (M(1, 0, 1) * M(1, 0, 1) + M(0, 1, 1) * M(0, 1, 1) + M(1, 1, 0) * M(1, 1, 0))
-                      + (M(0, 0, 2) * M(0, 2, 0) + M(0, 0, 2) * M(2, 0, 0) + M(0, 2, 0) * M(2, 0, 0)) + c13 * (M(0, 0, 2) + M(0, 2, 0) + M(2, 0, 0))) * r2 * c23
-                   + c127 * ((drho * drho - drho) * r2));
-
-    M(1, 0, 0) = -M(1, 0, 0);
-    M(0, 1, 0) = -M(0, 1, 0);
-    M(0, 0, 1) = -M(0, 0, 1);
-
-    const T x2mv = vx2 - vx, x2pv = vx2 + vx, y2mv = vy2 - vy, y2pv = vy2 + vy, z2mv = vz2 - vz, z2pv = vz2 + vz;
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const T K = (b == 0 && c == 0) ? T(1) : (b == 2 && c == 2) ? T(1) / T(9)
-                      : ((b == 2 && c == 0) || (b == 0 && c == 2)) ? T(1) / T(3) : T(0);
-            bwdK(M(0, b, c), M(1, b, c), M(2, b, c), vx, x2mv, x2pv, twovx, vx2, K);
+            const T a0 = M(0, b, c);
+            const T w = b == 1 || c == 1 ? a0 : a0 + T(b + c == 0 ? B(1) : b + c == 2 ? B(1) / B(3) : B(1) / B(9));
+            back_line(M(0, b, c), M(1, b, c), M(2, b, c), vx, vx2, twovx, w, half, mhalf);
         }
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-            bwdK(M(a, 0, c), M(a, 1, c), M(a, 2, c), vy, y2mv, y2pv, twovy, vy2, c == 1 ? T(0) : k_y<T>(a, c));
+        for (int c = 0; c < 3; ++c) {
+            const T a0 = M(a, 0, c);
+            const T w = c == 1 ? a0 : a0 + T(k_y<B>(a, c));
+            back_line(M(a, 0, c), M(a, 1, c), M(a, 2, c), vy, vy2, twovy, w, half, mhalf);
+        }
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int b = 0; b < 3; ++b)
-            bwdK(M(a, b, 0), M(a, b, 1), M(a, b, 2), vz, z2mv, z2pv, twovz, vz2, k_z<T>(a, b));
+            back_line(M(a, b, 0), M(a, b, 1), M(a, b, 2), vz, vz2, twovz, M(a, b, 0) + T(k_z<B>(a, b)), half, mhalf);
 #undef M
 
 #pragma unroll
@@ -715,9 +707,21 @@ namespace vfb {
 template <class T, bool EXACT>
 __host__ __device__ __forceinline__ void collide(T *f, const K17Rates<T> &r, T fx, T fy, T fz, T &drho, T &vx, T &vy, T &vz)
 {
-    if constexpr (EXACT)
+    if constexpr (EXACT) {
         k17_collide<T, true>(f, r, fx, fy, fz, drho, vx, vy, vz);
-    else
-        k17_collide_fast<T>(f, make_k17_fast_const(r), fx, fy, fz, drho, vx, vy, vz);
+    } else {
+        Rn<T> g[27], out[4];
+#pragma unroll
+        for (int d = 0; d < 27; ++d)
+            g[d] = f[d];
+        k17_collide_fast<Rn<T>, T>(g, r, fx, fy, fz, out[0], out[1], out[2], out[3]);
+#pragma unroll
+        for (int d = 0; d < 27; ++d)
+            f[d] = g[d].v;
+        drho = out[0].v;
+        vx = out[1].v;
+        vy = out[2].v;
+        vz = out[3].v;
+    }
 }
 } // namespace vfb

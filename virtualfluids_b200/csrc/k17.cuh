@@ -452,6 +452,7 @@ template <class B> inline B rn_fma(B a, B b, B c) { return std::fma(a, b, c); }
 template <class B> __host__ __device__ __forceinline__ Rn<B> operator+(Rn<B> a, Rn<B> b) { return rn_add(a.v, b.v); }
 template <class B> __host__ __device__ __forceinline__ Rn<B> operator-(Rn<B> a, Rn<B> b) { return rn_add(a.v, -b.v); }
 template <class B> __host__ __device__ __forceinline__ Rn<B> operator*(Rn<B> a, Rn<B> b) { return rn_mul(a.v, b.v); }
+template <class B> __host__ __device__ __forceinline__ Rn<B> operator/(Rn<B> a, Rn<B> b) { return a.v / b.v; }
 template <class B> __host__ __device__ __forceinline__ Rn<B> operator-(Rn<B> a) { return Rn<B>(-a.v); }
 template <class B> __host__ __device__ __forceinline__ Rn<B> fma(Rn<B> a, Rn<B> b, Rn<B> c) { return rn_fma(a.v, b.v, c.v); }
 

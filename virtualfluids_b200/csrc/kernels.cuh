@@ -968,6 +968,18 @@ __device__ __forceinline__ bool q_active(C q)
     return q >= C(0) && q <= C(1);
 }
 
+// The q of a BC node's 26 links, all loaded before the node's first store: the stores may alias the
+// list as far as the compiler can tell, so a q read in the loop over the links waits for the links
+// before it (26 memory latencies in a row: 16 us for any list, however short).
+template <class C>
+__device__ __forceinline__ void load_link_q(const C *__restrict__ q27, uint64_t stride, C (&q)[27])
+{
+    q[0] = C(-1);
+#pragma unroll
+    for (int d = 1; d < 27; ++d)
+        q[d] = __ldg(q27 + (uint64_t)d * stride);
+}
+
 // NoSlipBounceBack_Device (NoSlip/NoSlipBounceBack.cu:44-179) and VelocityBounceBack_Device
 // (Velocity/VelocityBounceBack.cu:44-188): for every link with q in [0,1] the population leaving
 // along d comes back as inv(d) into the slot the node reads on the next step; the velocity
@@ -1000,7 +1012,8 @@ __global__ void __launch_bounds__(128) bc_bounce_back_kernel(BCArgs a)
                     post[d] = saved[r++];
         }
     }
-    const C *q27 = static_cast<const C *>(a.q27);
+    C q[27];
+    load_link_q(static_cast<const C *>(a.q27) + i, a.nbc, q);
     C ux = C(0), uy = C(0), uz = C(0);
     if (VELOCITY) {
         ux = static_cast<const C *>(a.ux)[i];
@@ -1009,8 +1022,7 @@ __global__ void __launch_bounds__(128) bc_bounce_back_kernel(BCArgs a)
     }
 #pragma unroll
     for (int d = 1; d < 27; ++d) {
-        const C q = q27[(uint64_t)d * a.nbc + i];
-        if (q_active(q)) {
+        if (q_active(q[d])) {
             const int e = inv(d);
             C v = post[d];
             if (VELOCITY) {
@@ -1071,6 +1083,18 @@ __device__ __forceinline__ C cdot_rt(int d, C ux, C uy, C uz)
 //                       links is cut.
 enum : int { kBCCompressible = 0, kBCIncompressible = 1, kBCWithPressure = 2, kBCSlip = 3 };
 
+// The BC values are formed from operations that each round on their own, with a product and a sum
+// fused where mad says so (never in the exact variant): a box, a pool and a list level run
+// different kernels over these helpers and compute the same bits, whatever code stands around them.
+template <class C>
+__device__ __forceinline__ Rn<C> mad(Rn<C> a, Rn<C> b, Rn<C> c)
+{
+    if constexpr (VFB_EXACT)
+        return a * b + c;
+    else
+        return fma(a, b, c);
+}
+
 // density, velocity and c_s^2-scaled u^2 of a BC node's post-collision populations
 // (NoSlipInterpolatedCompressible.cu:134-153: plain-sum density, grouped momenta)
 template <class C>
@@ -1081,44 +1105,47 @@ struct BCMoments {
 template <class C, int FORM>
 __device__ __forceinline__ BCMoments<C> bc_moments(const C (&p)[27])
 {
+    using R = Rn<C>;
     BCMoments<C> m;
     m.drho = p[21] + p[20] + p[19] + p[22] + p[25] + p[24] + p[23] + p[26] + p[17] + p[18] + p[15] + p[16] + p[13]
            + p[14] + p[11] + p[12] + p[9] + p[10] + p[7] + p[8] + p[5] + p[6] + p[3] + p[4] + p[1] + p[2] + p[0];
-    const C r = C(1) + m.drho;
+    const R r = R(C(1)) + R(m.drho);
     const C vx = (((((p[21] - p[24]) - (p[20] - p[25])) + ((p[19] - p[26]) - (p[22] - p[23]))) + ((p[13] - p[14]) + (p[11] - p[12])))
                   + ((p[9] - p[10]) + (p[7] - p[8]))) + (p[1] - p[2]);
     const C vy = (((((-(p[21] - p[24])) + (p[20] - p[25])) + ((p[19] - p[26]) - (p[22] - p[23]))) + ((p[17] - p[18]) + (p[15] - p[16])))
                   + ((-(p[9] - p[10])) + (p[7] - p[8]))) + (p[3] - p[4]);
     const C vz = (((((p[21] - p[24]) + (p[20] - p[25])) + ((p[19] - p[26]) + (p[22] - p[23]))) + ((-(p[17] - p[18])) + (p[15] - p[16])))
                   + ((p[11] - p[12]) - (p[13] - p[14]))) + (p[5] - p[6]);
-    m.ux = FORM == kBCIncompressible ? vx : vx / r;
-    m.uy = FORM == kBCIncompressible ? vy : vy / r;
-    m.uz = FORM == kBCIncompressible ? vz : vz / r;
-    m.cu_sq = FORM == kBCIncompressible ? C(1.5) * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz)
-                                        : C(1.5) * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz) * (C(1) + m.drho);
+    const R ux = FORM == kBCIncompressible ? R(vx) : R(vx) / r;
+    const R uy = FORM == kBCIncompressible ? R(vy) : R(vy) / r;
+    const R uz = FORM == kBCIncompressible ? R(vz) : R(vz) / r;
+    const R c = R(C(1.5)) * mad(uz, uz, mad(uy, uy, ux * ux));
+    m.ux = ux.v;
+    m.uy = uy.v;
+    m.uz = uz.v;
+    m.cu_sq = FORM == kBCIncompressible ? c.v : (c * r).v;
     return m;
 }
 
 // the value written for one cut link: f = p[d], fi = p[inv d], w and vel = c_d . u of direction d,
 // vbc = c_d . u_wall (velocity kernels)
 template <class C, bool VELOCITY, int FORM>
-__device__ __forceinline__ C bc_link_value(C f, C fi, C q, C w, C vel, C vbc, const BCMoments<C> &m, C omega)
+__device__ __forceinline__ C bc_link_value(C f_, C fi_, C q_, C w_, C vel_, C vbc, const BCMoments<C> &m, C omega_)
 {
+    using R = Rn<C>;
+    const R f = f_, fi = fi_, q = q_, w = w_, vel = vel_, omega = omega_, drho = m.drho, one = C(1);
     // the incompressible velocity kernel writes feq inline without (1 + drho); the incompressible
     // no-slip kernel keeps getEquilibriumForBC, which carries it
-    const C feq = (FORM == kBCIncompressible && VELOCITY) ? w * (m.drho + C(4.5) * vel * vel - m.cu_sq)
-                                                          : w * (m.drho + C(4.5) * vel * vel * (C(1) + m.drho) - m.cu_sq);
-    C v;
-    if (VELOCITY) {
-        v = (C(1) - q) / (C(1) + q) * (f - fi + (f + fi - C(2) * feq * omega) / (C(1) - omega)) * C(0.5)
-          + (q * (f + fi) - C(6) * w * vbc) / (C(1) + q);
-        if (FORM == kBCWithPressure)
-            v = v - w * m.drho;
-    } else {
-        v = (C(1) - q) / (C(1) + q) * (f - fi + (f + fi - C(2) * feq * omega) / (C(1) - omega)) * C(0.5)
-          + (q * (f + fi)) / (C(1) + q);
-    }
-    return v;
+    const R v45 = R(C(4.5)) * vel;
+    const R feq = w * (((FORM == kBCIncompressible && VELOCITY) ? mad(v45, vel, drho) : mad(v45 * vel, one + drho, drho))
+                       - R(m.cu_sq));
+    const R s = f + fi;
+    const R part = (one - q) / (one + q) * (f - fi + mad(-(R(C(2)) * feq), omega, s) / (one - omega));
+    const R wall = VELOCITY ? mad(q, s, -(R(C(6)) * w * R(vbc))) : q * s;
+    R v = mad(part, R(C(0.5)), wall / (one + q));
+    if (VELOCITY && FORM == kBCWithPressure)
+        v = mad(-w, drho, v);
+    return v.v;
 }
 
 // one BC node: its slot nodes, its q of every direction at q27[d * q_stride], the wall velocity
@@ -1132,7 +1159,8 @@ __device__ __forceinline__ void bc_interpolated_node(S *base, uint64_t n, const 
                                                      const typename Codec<S>::compute *guard = nullptr)
 {
     using C = typename Codec<S>::compute;
-    C p[27];
+    C p[27], q[27];
+    load_link_q(q27, q_stride, q);
     if (snap) {
 #pragma unroll
         for (int d = 0; d < 27; ++d)
@@ -1153,18 +1181,17 @@ __device__ __forceinline__ void bc_interpolated_node(S *base, uint64_t n, const 
     if (FORM == kBCSlip) {
         // the reference zeroes VeloX when the link P00 or M00 is cut, and so on; the links along the
         // axes come first there, so every diagonal link sees the zeroing of all three axes
-        const bool cut_x = q_active(q27[1 * q_stride]) || q_active(q27[2 * q_stride]);
-        const bool cut_y = q_active(q27[3 * q_stride]) || q_active(q27[4 * q_stride]);
-        const bool cut_z = q_active(q27[5 * q_stride]) || q_active(q27[6 * q_stride]);
+        const bool cut_x = q_active(q[1]) || q_active(q[2]);
+        const bool cut_y = q_active(q[3]) || q_active(q[4]);
+        const bool cut_z = q_active(q[5]) || q_active(q[6]);
         bx = cut_x ? C(0) : m.ux;
         by = cut_y ? C(0) : m.uy;
         bz = cut_z ? C(0) : m.uz;
     }
 #pragma unroll
     for (int d = 1; d < 27; ++d) {
-        const C q = q27[(uint64_t)d * q_stride];
-        if (q_active(q)) {
-            const C v = bc_link_value<C, VELOCITY, FORM>(p[d], p[inv(d)], q, weight_t<C>(d), cdot_rt<C>(d, m.ux, m.uy, m.uz),
+        if (q_active(q[d])) {
+            const C v = bc_link_value<C, VELOCITY, FORM>(p[d], p[inv(d)], q[d], weight_t<C>(d), cdot_rt<C>(d, m.ux, m.uy, m.uz),
                                                          VELOCITY ? cdot_rt<C>(d, bx, by, bz) : C(0), m, omega);
             const int e = inv(d);
             Codec<S>::store_at(base, (uint64_t)plane<!EVEN>(e) * n + nodes[shift_class(e)], v, e);
@@ -1195,6 +1222,24 @@ __global__ void __launch_bounds__(128) bc_interpolated_kernel(BCArgs a)
                                                   snap, a.nbc, mask, saved);
 }
 
+// one node's guarded post-collision values, in the order of their directions; every value is loaded
+// before the first is stored (a load behind a store that may alias it waits for the store's own load)
+template <class S, bool EVEN>
+__device__ __forceinline__ void save_guarded(const S *__restrict__ base, uint64_t n, const uint32_t (&nodes)[8],
+                                             uint32_t mask, typename Codec<S>::compute *__restrict__ out)
+{
+    typename Codec<S>::compute v[27];
+#pragma unroll
+    for (int d = 1; d < 27; ++d)
+        if ((mask >> d) & 1u)
+            v[d] = Codec<S>::load(base + (uint64_t)plane<EVEN>(inv(d)) * n + nodes[shift_class(inv(d))], d);
+    int r = 0;
+#pragma unroll
+    for (int d = 1; d < 27; ++d)
+        if ((mask >> d) & 1u)
+            out[r++] = v[d];
+}
+
 // the guarded post-collision values of a list (guards.h), saved before the list's BC kernel writes
 template <class S, bool EVEN>
 __global__ void __launch_bounds__(128) bc_guard_kernel(BCArgs a, typename Codec<S>::compute *saved)
@@ -1207,13 +1252,7 @@ __global__ void __launch_bounds__(128) bc_guard_kernel(BCArgs a, typename Codec<
         return;
     uint32_t nodes[8];
     node_slots((uint32_t)a.k[i], a.nbx, a.nby, a.nbz, a.n, a.box, nodes);
-    const S *base = static_cast<const S *>(a.dist);
-    typename Codec<S>::compute *out = saved + a.guard[a.nbc + i];
-    int r = 0;
-#pragma unroll
-    for (int d = 1; d < 27; ++d)
-        if ((mask >> d) & 1u)
-            out[r++] = Codec<S>::load(base + (uint64_t)plane<EVEN>(inv(d)) * a.n + nodes[shift_class(inv(d))], d);
+    save_guarded<S, EVEN>(static_cast<const S *>(a.dist), a.n, nodes, mask, saved + a.guard[a.nbc + i]);
 }
 
 // The post-collision populations of every node of a BC list into snap[d * nbc + i], taken before
@@ -1236,14 +1275,15 @@ __global__ void __launch_bounds__(128) bc_snapshot_kernel(BCArgs a, typename Cod
         snap[(uint64_t)d * a.nbc + i] = p[d];
 }
 
-// feq - w of one direction in the form of the init and pressure kernels
+// (feq - w) / w of one direction in the form of the pressure kernels, cu = c_d . u
 template <class C>
-__device__ __forceinline__ C feq_shifted(int d, C drho, C ux, C uy, C uz, C cusq)
+__device__ __forceinline__ Rn<C> feq_over_w(int d, Rn<C> drho, C cu_, Rn<C> cusq)
 {
+    using R = Rn<C>;
+    const R rho = drho + R(C(1)), cu = cu_;
     if (d == 0)
-        return weight_t<C>(0) * (drho - (drho + C(1)) * cusq);
-    const C cu = cdot_rt<C>(d, ux, uy, uz);
-    return weight_t<C>(d) * (drho + (drho + C(1)) * (C(3) * cu + C(4.5) * cu * cu - cusq));
+        return mad(-rho, cusq, drho);
+    return mad(rho, mad(R(C(4.5)) * cu, cu, R(C(3)) * cu) - cusq, drho);
 }
 
 // PressureNonEquilibriumCompressible_Device (Pressure/PressureNonEquilibriumCompressible.cu:45-314).
@@ -1261,28 +1301,21 @@ __device__ __forceinline__ void bc_pressure_neq_node(S *base, uint64_t n, const 
     using C = typename Codec<S>::compute;
     C f[27];
     gather_pre<S, EVEN>(base, n, nn, f);
-    const C drho1 = density_pyramid(f);
-    C vx, vy, vz;
-    if (INCOMP) {
-        vx = momentum_x(f);
-        vy = momentum_y(f);
-        vz = momentum_z(f);
-    } else {
-        const C inv_rho = C(1) / (drho1 + C(1));
-        vx = momentum_x(f) * inv_rho;
-        vy = momentum_y(f) * inv_rho;
-        vz = momentum_z(f) * inv_rho;
-    }
-    const C cusq = C(1.5) * (vx * vx + vy * vy + vz * vz);
+    using R = Rn<C>;
+    const R drho1 = density_pyramid(f);
+    const R inv_rho = INCOMP ? R(C(1)) : R(C(1)) / (drho1 + R(C(1)));
+    const R vx = R(momentum_x(f)) * inv_rho, vy = R(momentum_y(f)) * inv_rho, vz = R(momentum_z(f)) * inv_rho;
+    const R cusq = R(C(1.5)) * mad(vz, vz, mad(vy, vy, vx * vx));
     const int axis = cx(direction) != 0 ? 0 : (cy(direction) != 0 ? 1 : 2);
     const int sgn = axis == 0 ? cx(direction) : (axis == 1 ? cy(direction) : cz(direction));
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
-        C v = f[d] - feq_shifted<C>(d, drho1, vx, vy, vz, cusq);
-        v = v + feq_shifted<C>(d, rbc, vx, vy, vz, cusq);
+        const C cu = d ? cdot_rt<C>(d, vx.v, vy.v, vz.v) : C(0);
+        const R w = weight_t<C>(d);
+        const R v = mad(w, feq_over_w<C>(d, rbc, cu, cusq), mad(-w, feq_over_w<C>(d, drho1, cu, cusq), R(f[d])));
         const int c = axis == 0 ? cx(d) : (axis == 1 ? cy(d) : cz(d));
         if (c != sgn)
-            Codec<S>::store_at(base, (uint64_t)plane<EVEN>(d) * n + nk[shift_class(d)], v, d);
+            Codec<S>::store_at(base, (uint64_t)plane<EVEN>(d) * n + nk[shift_class(d)], v.v, d);
     }
 }
 
@@ -2093,12 +2126,7 @@ __global__ void __launch_bounds__(128) pool_noslip_guard_kernel(PoolBCArgs<typen
         const NodeAddr box{ dm.nx, dm.ny, dm.nz, dm.flags & 7 };
         uint32_t nodes[8];
         box_nodes((uint32_t)k[i], box, dm.div_nx, dm.div_ny, nodes);
-        const S *base = static_cast<const S *>(a.arena) + dm.dist_offset;
-        int r = 0;
-#pragma unroll
-        for (int d = 1; d < 27; ++d)
-            if ((mask >> d) & 1u)
-                saved[r++] = Codec<S>::load(base + (uint64_t)plane<EVEN>(inv(d)) * dm.pitch + nodes[shift_class(inv(d))], d);
+        save_guarded<S, EVEN>(static_cast<const S *>(a.arena) + dm.dist_offset, dm.pitch, nodes, mask, saved);
     }
 }
 

@@ -180,6 +180,60 @@ template <class T> __host__ __device__ __forceinline__ T k_y(int a, int c)
     return a != 1 ? (c == 0 ? T(1) / T(6) : T(1) / T(18)) : (c == 0 ? T(2) / T(3) : T(2) / T(9));
 }
 
+// Correctly rounded 1 / b and a / b in double without a branch, b > 0 (an infinity or NaN in a or b
+// gives NaN). Method: Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34 (1990); Cornea, Harrison, Tang, "Scientific Computing on Itanium-based
+// Systems" (2002), ch. 8:
+//  * y1 is within one unit in the last place of 1 / b: the hardware's approximation refined by one
+//    cubic step (its error, below 2^-18, to the third power is far below the rounding of y1);
+//  * then y2 = y1 + y1 (1 - b y1), one rounding, is the rounded reciprocal, except where b's 52
+//    fraction bits are all ones: y2 may be a power of two there, and the rounded reciprocal is
+//    the next double (its last bit set);
+//  * with y2 the rounded reciprocal, q1 = q0 + y2 (a - b q0), one rounding, is the rounded quotient
+//    (the remainder is exact).
+// It holds for b in [2^-1000, 2^1021] and quotients above 2^-960. The exact collision divides by
+// |m| + q with the limiter q, and by 1 + drho; a smaller quotient is added to a rate or multiplied
+// onto a moment that it cannot change. The compiler's division has a branch to a slow path in
+// each of the eight, between which no arithmetic moves.
+__host__ __device__ __forceinline__ double refine_rcp(double b, double y)
+{
+    const double e = ::fma(-b, y, 1.0);
+    y = ::fma(y, ::fma(e, e, e), y);
+    y = ::fma(y, ::fma(-b, y, 1.0), y);
+#ifdef __CUDA_ARCH__
+    const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
+    return __hiloint2double(__double2hiint(y), __double2loint(y) | ((lo & (hi | 0xfff00000u)) == 0xffffffffu ? 1 : 0));
+#else
+    uint64_t bits, r;
+    __builtin_memcpy(&bits, &b, 8);
+    __builtin_memcpy(&r, &y, 8);
+    r |= (~bits & 0xfffffffffffffull) == 0 ? 1 : 0;
+    __builtin_memcpy(&y, &r, 8);
+    return y;
+#endif
+}
+__host__ __device__ __forceinline__ double refine_div(double a, double b, double y)
+{
+    y = refine_rcp(b, y);
+    const double q = a * y;
+    return ::fma(::fma(-b, q, a), y, q);
+}
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ double rcp_seed(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    return y;
+}
+__device__ __forceinline__ double rcp_rounded(double b) { return refine_rcp(b, rcp_seed(b)); }
+__device__ __forceinline__ double div_rounded(double a, double b) { return refine_div(a, b, rcp_seed(b)); }
+#else
+inline double rcp_rounded(double b) { return 1.0 / b; }
+inline double div_rounded(double a, double b) { return a / b; }
+#endif
+__host__ __device__ __forceinline__ float rcp_rounded(float b) { return 1.0f / b; }
+__host__ __device__ __forceinline__ float div_rounded(float a, float b) { return a / b; }
+
 } // namespace k17detail
 
 // pyramid density (MacroscopicQuantities.h:55), f in direction order
@@ -221,7 +275,7 @@ __host__ __device__ __forceinline__ void k17_collide(T *f, const K17Rates<T> &r,
 {
     using namespace k17detail;
     const T drho = density_pyramid(f);
-    const T oneOverRho = T(1) / (drho + T(1));
+    const T oneOverRho = rcp_rounded(drho + T(1));
     T vx = momentum_x(f) * oneOverRho;
     T vy = momentum_y(f) * oneOverRho;
     T vz = momentum_z(f) * oneOverRho;
@@ -298,19 +352,19 @@ __host__ __device__ __forceinline__ void k17_collide(T *f, const K17Rates<T> &r,
 
     // third order with the quartic limiter (K17...h:397-410)
     T wadj;
-    wadj = r.Oxyz + r.omOxyz * fabs(M(1, 1, 1)) / (fabs(M(1, 1, 1)) + r.qD);
+    wadj = r.Oxyz + div_rounded(r.omOxyz * fabs(M(1, 1, 1)), fabs(M(1, 1, 1)) + r.qD);
     M(1, 1, 1) += wadj * (-M(1, 1, 1));
-    wadj = r.OxyyPxzz + r.omOP * fabs(mxxyPyzz) / (fabs(mxxyPyzz) + r.qP);
+    wadj = r.OxyyPxzz + div_rounded(r.omOP * fabs(mxxyPyzz), fabs(mxxyPyzz) + r.qP);
     mxxyPyzz += wadj * (-mxxyPyzz);
-    wadj = r.OxyyMxzz + r.omOM * fabs(mxxyMyzz) / (fabs(mxxyMyzz) + r.qM);
+    wadj = r.OxyyMxzz + div_rounded(r.omOM * fabs(mxxyMyzz), fabs(mxxyMyzz) + r.qM);
     mxxyMyzz += wadj * (-mxxyMyzz);
-    wadj = r.OxyyPxzz + r.omOP * fabs(mxxzPyyz) / (fabs(mxxzPyyz) + r.qP);
+    wadj = r.OxyyPxzz + div_rounded(r.omOP * fabs(mxxzPyyz), fabs(mxxzPyyz) + r.qP);
     mxxzPyyz += wadj * (-mxxzPyyz);
-    wadj = r.OxyyMxzz + r.omOM * fabs(mxxzMyyz) / (fabs(mxxzMyyz) + r.qM);
+    wadj = r.OxyyMxzz + div_rounded(r.omOM * fabs(mxxzMyyz), fabs(mxxzMyyz) + r.qM);
     mxxzMyyz += wadj * (-mxxzMyyz);
-    wadj = r.OxyyPxzz + r.omOP * fabs(mxyyPxzz) / (fabs(mxyyPxzz) + r.qP);
+    wadj = r.OxyyPxzz + div_rounded(r.omOP * fabs(mxyyPxzz), fabs(mxyyPxzz) + r.qP);
     mxyyPxzz += wadj * (-mxyyPxzz);
-    wadj = r.OxyyMxzz + r.omOM * fabs(mxyyMxzz) / (fabs(mxyyMxzz) + r.qM);
+    wadj = r.OxyyMxzz + div_rounded(r.omOM * fabs(mxyyMxzz), fabs(mxyyMxzz) + r.qM);
     mxyyMxzz += wadj * (-mxyyMxzz);
 
     // back from the linear combinations (K17...h:424-433)

@@ -1081,7 +1081,7 @@ static vfb::BoxState regular_box_state(const SimLevel &S)
     b.fz = list_half_force(L, 2);
     for (int i = 0; i < 3; ++i)
         b.lim[i] = L.quadric_limiters[i];
-    b.variant = 1;
+    b.variant = 0;
     b.status = nullptr;
     return b;
 }

@@ -11,6 +11,9 @@ struct NodeAddr {
     int nx, ny, nz, periodic;
 };
 
+// whether a direction plane of `nodes` nodes can be addressed with 32-bit byte offsets (slot_at)
+inline bool narrow_planes(uint64_t nodes, uint64_t storage_bytes) { return nodes * storage_bytes < (1ull << 32); }
+
 // Division by a run-time constant d in [1, 2^16) of dividends n < 2^31 with one wide multiply and a
 // shift (Granlund and Montgomery, "Division by invariant integers using multiplication", PLDI
 // 1994): with l = ceil(log2 d) and m = ceil(2^(31+l) / d) < 2^32, floor(n / d) = (n m) >> (31 + l),

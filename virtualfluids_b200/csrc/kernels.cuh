@@ -76,7 +76,11 @@ struct BoxCollideArgs {
     C fx, fy, fz;
     double *energy_partials;    // optional: per block {sum(1+drho), sum(0.5 (1+drho) u^2)}
     C *rho, *vx, *vy, *vz;      // optional macroscopic outputs
-    int z_begin;                // the direct kernel collides planes z_begin + blockIdx.z (0: the whole box)
+    // the node range [first, first + count) of the one- and two-node kernels, and their index
+    // arithmetic: multiply-shifts where `exact_div` holds (addr.h), else hardware division
+    uint32_t first, count;
+    FastDiv div_nx, div_ny;
+    int exact_div;
 };
 
 // where a node's eight slot nodes are: from the neighbour lists (reference layout), or, when
@@ -179,17 +183,17 @@ __device__ __forceinline__ void node_slots(uint32_t k, const uint32_t *nbx, cons
         box_nodes(k, b, nodes);
 }
 
-template <class S, bool EVEN>
+template <class S, bool EVEN, bool NARROW = false>
 __device__ __forceinline__ void gather_pre(const S *__restrict__ base, uint64_t n, const uint32_t (&nodes)[8],
                                            typename Codec<S>::compute (&f)[27])
 {
 #pragma unroll
     for (int d = 0; d < 27; ++d)
-        f[d] = Codec<S>::load(base + (uint64_t)plane<EVEN>(d) * n + nodes[shift_class(d)], d);
+        f[d] = Codec<S>::load(slot_at<NARROW>(base + (uint64_t)plane<EVEN>(d) * n, nodes[shift_class(d)]), d);
 }
 
 // setPostCollisionDistribution (KernelUtilities.h:350): the slot of d receives f[inv d]
-template <class S, bool EVEN>
+template <class S, bool EVEN, bool NARROW = false>
 __device__ __forceinline__ void scatter_post(S *__restrict__ base, uint64_t n, const uint32_t (&nodes)[8],
                                              const typename Codec<S>::compute (&f)[27])
 {
@@ -197,13 +201,14 @@ __device__ __forceinline__ void scatter_post(S *__restrict__ base, uint64_t n, c
         // 16-bit storage: two directions share one stochastic-rounding conversion
 #pragma unroll
         for (int d = 0; d + 1 < 27; d += 2)
-            Codec<S>::store_pair_at(base, (uint64_t)plane<EVEN>(d) * n + nodes[shift_class(d)], f[inv(d)], d,
-                                    (uint64_t)plane<EVEN>(d + 1) * n + nodes[shift_class(d + 1)], f[inv(d + 1)], d + 1);
+            Codec<S>::template store_pair<NARROW>(base + (uint64_t)plane<EVEN>(d) * n, nodes[shift_class(d)],
+                                 (uint32_t)((uint64_t)plane<EVEN>(d) * n), f[inv(d)], d,
+                                 base + (uint64_t)plane<EVEN>(d + 1) * n, nodes[shift_class(d + 1)], f[inv(d + 1)], d + 1);
         Codec<S>::store_at(base, (uint64_t)plane<EVEN>(26) * n + nodes[shift_class(26)], f[inv(26)], 26);
     } else {
 #pragma unroll
         for (int d = 0; d < 27; ++d)
-            Codec<S>::store_at(base, (uint64_t)plane<EVEN>(d) * n + nodes[shift_class(d)], f[inv(d)], d);
+            Codec<S>::store(slot_at<NARROW>(base + (uint64_t)plane<EVEN>(d) * n, nodes[shift_class(d)]), f[inv(d)], d);
     }
 }
 
@@ -355,7 +360,9 @@ __global__ void __launch_bounds__(128) k17_list_staged_kernel(ListCollideArgs<ty
 
 // ---------------------------------------------------------------------------------------------
 // collision + streaming on a structured box: neighbours by index arithmetic, one node per
-// thread, x fastest so every direction plane is read and written by whole warps in order.
+// thread, threads in node order (x fastest) through the whole box, so every direction plane is read
+// and written by full warps in order whatever the row length. A grid of 128-thread blocks along
+// each row left part of the last block of a row without nodes but not without registers.
 // ---------------------------------------------------------------------------------------------
 // resident blocks per SM the register budget must allow: three for FP64 arithmetic (at most 168
 // registers; an unbounded build of the exact energy variant takes 170, which rounds to 176 and
@@ -363,68 +370,67 @@ __global__ void __launch_bounds__(128) k17_list_staged_kernel(ListCollideArgs<ty
 template <class S>
 constexpr int box_min_blocks() { return sizeof(typename Codec<S>::compute) == 8 ? 3 : 4; }
 
-template <class S, bool EXACT, bool EVEN, bool MASK, bool ENERGY, bool WRITE_MACRO>
+// the slot nodes of node k: +1 neighbours, wrapping on periodic axes (the mask keeps walled boxes inside)
+template <class C>
+__device__ __forceinline__ void box_slots(const BoxCollideArgs<C> &a, uint32_t k, uint32_t (&nodes)[8])
+{
+    const uint32_t nx = (uint32_t)a.nx, ny = (uint32_t)a.ny;
+    const uint32_t yz = a.exact_div ? fast_div(k, a.div_nx) : k / nx;
+    const uint32_t z = a.exact_div ? fast_div(yz, a.div_ny) : yz / ny;
+    const uint32_t x = k - yz * nx, y = yz - z * ny;
+    const uint32_t plane_nodes = nx * ny;
+    const uint32_t sx = x + 1 < nx ? 1u : a.periodic_x ? 1u - nx : 0u;
+    const uint32_t sy = y + 1 < ny ? nx : a.periodic_y ? nx - plane_nodes : 0u;
+    const uint32_t sz = z + 1 < (uint32_t)a.nz ? plane_nodes : a.periodic_z ? (1u - (uint32_t)a.nz) * plane_nodes : 0u;
+    nodes[0] = k;
+    nodes[1] = k + sx;
+    nodes[2] = k + sy;
+    nodes[3] = k + sx + sy;
+    nodes[4] = k + sz;
+    nodes[5] = k + sx + sz;
+    nodes[6] = k + sy + sz;
+    nodes[7] = k + sx + sy + sz;
+}
+
+// FP64 partials of mass and kinetic energy per warp (fixed reduction order, no block barrier, so the
+// warps of a block retire independently)
+__device__ __forceinline__ void store_energy_partial(double *partials, double m, double e)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        m += __shfl_down_sync(0xffffffffu, m, o);
+        e += __shfl_down_sync(0xffffffffu, e, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        const uint64_t w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        partials[2 * w] = m;
+        partials[2 * w + 1] = e;
+    }
+}
+
+template <class S, bool EXACT, bool EVEN, bool MASK, bool ENERGY, bool NARROW>
 __global__ void __launch_bounds__(128, box_min_blocks<S>()) k17_box_kernel(BoxCollideArgs<typename Codec<S>::compute> a)
 {
     using C = typename Codec<S>::compute;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y;
-    const int z = blockIdx.z + a.z_begin;
-    const bool active_x = x < a.nx;
-    const uint64_t row = (uint64_t)a.nx * ((uint64_t)y + (uint64_t)a.ny * (uint64_t)z);
-    const uint32_t k = (uint32_t)(row + (uint64_t)x);
-    bool active = active_x;
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t k = a.first + (uint32_t)i;
+    bool active = i < a.count;
     if (MASK && active)
         active = __ldg(a.mask + k) != 0;
 
     C drho = C(0), vx = C(0), vy = C(0), vz = C(0);
     if (active) {
-        // +1 neighbours, wrapping on periodic axes (the mask keeps walled boxes inside)
-        const int xp = (x + 1 < a.nx) ? x + 1 : (a.periodic_x ? 0 : x);
-        const int yp = (y + 1 < a.ny) ? y + 1 : (a.periodic_y ? 0 : y);
-        const int zp = (z + 1 < a.nz) ? z + 1 : (a.periodic_z ? 0 : z);
-        const uint32_t sx = (uint32_t)(xp - x);
-        const uint32_t sy = (uint32_t)((yp - y) * a.nx);
-        const uint32_t sz = (uint32_t)((int64_t)(zp - z) * a.nx * a.ny);
         uint32_t nodes[8];
-        nodes[0] = k;
-        nodes[1] = k + sx;
-        nodes[2] = k + sy;
-        nodes[3] = k + sx + sy;
-        nodes[4] = k + sz;
-        nodes[5] = k + sx + sz;
-        nodes[6] = k + sy + sz;
-        nodes[7] = k + sx + sy + sz;
+        box_slots(a, k, nodes);
         S *base = static_cast<S *>(a.dist);
         C f[27];
-        gather_pre<S, EVEN>(base, a.pitch, nodes, f);
+        gather_pre<S, EVEN, NARROW>(base, a.pitch, nodes, f);
         collide<C, EXACT>(f, a.rates, a.fx, a.fy, a.fz, drho, vx, vy, vz);
-        if (WRITE_MACRO) {
-            a.rho[k] = drho;
-            a.vx[k] = vx;
-            a.vy[k] = vy;
-            a.vz[k] = vz;
-        }
-        scatter_post<S, EVEN>(base, a.pitch, nodes, f);
+        scatter_post<S, EVEN, NARROW>(base, a.pitch, nodes, f);
     }
-
-    if (ENERGY) {
-        // FP64 partials of mass and kinetic energy per warp (fixed reduction order, no block barrier,
-        // so the warps of a block retire independently)
-        double m = active ? 1.0 + (double)drho : 0.0;
-        double e = active ? 0.5 * (1.0 + (double)drho) * ((double)vx * vx + (double)vy * vy + (double)vz * vz) : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            m += __shfl_down_sync(0xffffffffu, m, o);
-            e += __shfl_down_sync(0xffffffffu, e, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            const uint64_t b = blockIdx.x + (uint64_t)gridDim.x * (blockIdx.y + (uint64_t)gridDim.y * blockIdx.z);
-            const uint64_t w = b * (blockDim.x >> 5) + (threadIdx.x >> 5);
-            a.energy_partials[2 * w] = m;
-            a.energy_partials[2 * w + 1] = e;
-        }
-    }
+    if (ENERGY)
+        store_energy_partial(a.energy_partials, active ? 1.0 + (double)drho : 0.0,
+                             active ? 0.5 * (1.0 + (double)drho) * ((double)vx * vx + (double)vy * vy + (double)vz * vz) : 0.0);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -590,58 +596,47 @@ __global__ void __launch_bounds__(128, pipe_min_blocks<S>()) k17_box_pipe_kernel
 }
 
 // ---------------------------------------------------------------------------------------------
-// The box collision for the FP32-arithmetic forms with two nodes per thread, (x, y) and (x, y + 1),
-// collided together in packed FP32x2 arithmetic (packed.cuh): the arithmetic issues about half the
-// instructions, the loads and stores stay coalesced per row. FMA arithmetic only.
+// The box collision for the FP32-arithmetic forms with two nodes per thread, 32 apart in node order
+// (a warp owns 64 consecutive nodes), collided together in packed FP32x2 arithmetic (packed.cuh):
+// the arithmetic issues half the instructions, every access stays a full warp's in order, and
+// each node's bits are those of k17_box_kernel. FMA arithmetic only. Bound: HBM and its latency
+// (FP32), issue and the FMA pipe (16-bit forms). Four blocks per SM (128 registers, no more than a
+// few spilled) beat three (150 registers): FP32 320 x 256 x 192 589 against 621 us per step, where
+// one node per thread takes 661; FP16 250 x 190 x 230 369 us against 412 with one node.
 // ---------------------------------------------------------------------------------------------
 template <class S, bool EVEN, bool MASK, bool ENERGY>
-__global__ void __launch_bounds__(128) k17_box_pair_kernel(BoxCollideArgs<float> a)
+__global__ void __launch_bounds__(128, 4) k17_box_pair_kernel(BoxCollideArgs<float> a)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int z = blockIdx.z;
-    const int y0 = 2 * (int)blockIdx.y;
+    const uint64_t i0 = 2ull * ((uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) + (threadIdx.x & 31u);
     bool act[2];
     uint32_t nodes[2][8];
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-        const int y = y0 + p;
-        const uint32_t k = (uint32_t)((uint64_t)a.nx * ((uint64_t)y + (uint64_t)a.ny * (uint64_t)z) + (uint64_t)x);
-        act[p] = x < a.nx && y < a.ny;
+        const uint64_t i = i0 + 32u * p;
+        const uint32_t k = a.first + (uint32_t)i;
+        act[p] = i < a.count;
         if (MASK && act[p])
             act[p] = __ldg(a.mask + k) != 0;
-        const int xp = (x + 1 < a.nx) ? x + 1 : (a.periodic_x ? 0 : x);
-        const int yp = (y + 1 < a.ny) ? y + 1 : (a.periodic_y ? 0 : y);
-        const int zp = (z + 1 < a.nz) ? z + 1 : (a.periodic_z ? 0 : z);
-        const uint32_t sx = (uint32_t)(xp - x);
-        const uint32_t sy = (uint32_t)((yp - y) * a.nx);
-        const uint32_t sz = (uint32_t)((int64_t)(zp - z) * a.nx * a.ny);
-        nodes[p][0] = k;
-        nodes[p][1] = k + sx;
-        nodes[p][2] = k + sy;
-        nodes[p][3] = k + sx + sy;
-        nodes[p][4] = k + sz;
-        nodes[p][5] = k + sx + sz;
-        nodes[p][6] = k + sy + sz;
-        nodes[p][7] = k + sx + sy + sz;
+        box_slots(a, k, nodes[p]);
     }
     float mac[2][4] = { { 0.f, 0.f, 0.f, 0.f }, { 0.f, 0.f, 0.f, 0.f } };
     if (act[0] || act[1]) {
         S *base = static_cast<S *>(a.dist);
         float fa[27], fb[27];
         // an inactive partner collides a rest state (drho = 0, u = 0): finite, never stored
-        if (act[0]) gather_pre<S, EVEN>(base, a.pitch, nodes[0], fa);
+        if (act[0]) gather_pre<S, EVEN, true>(base, a.pitch, nodes[0], fa);
         else
 #pragma unroll
             for (int d = 0; d < 27; ++d) fa[d] = 0.f;
-        if (act[1]) gather_pre<S, EVEN>(base, a.pitch, nodes[1], fb);
+        if (act[1]) gather_pre<S, EVEN, true>(base, a.pitch, nodes[1], fb);
         else
 #pragma unroll
             for (int d = 0; d < 27; ++d) fb[d] = 0.f;
         collide_pair(fa, fb, a.rates, a.fx, a.fy, a.fz, mac[0], mac[1]);
         if (act[0])
-            scatter_post<S, EVEN>(base, a.pitch, nodes[0], fa);
+            scatter_post<S, EVEN, true>(base, a.pitch, nodes[0], fa);
         if (act[1])
-            scatter_post<S, EVEN>(base, a.pitch, nodes[1], fb);
+            scatter_post<S, EVEN, true>(base, a.pitch, nodes[1], fb);
     }
     if (ENERGY) {
         double m = 0.0, e = 0.0;
@@ -652,17 +647,7 @@ __global__ void __launch_bounds__(128) k17_box_pair_kernel(BoxCollideArgs<float>
                 m += r;
                 e += 0.5 * r * ((double)mac[p][1] * mac[p][1] + (double)mac[p][2] * mac[p][2] + (double)mac[p][3] * mac[p][3]);
             }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            m += __shfl_down_sync(0xffffffffu, m, o);
-            e += __shfl_down_sync(0xffffffffu, e, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            const uint64_t b = blockIdx.x + (uint64_t)gridDim.x * (blockIdx.y + (uint64_t)gridDim.y * blockIdx.z);
-            const uint64_t w = b * (blockDim.x >> 5) + (threadIdx.x >> 5);
-            a.energy_partials[2 * w] = m;
-            a.energy_partials[2 * w + 1] = e;
-        }
+        store_energy_partial(a.energy_partials, m, e);
     }
 }
 
@@ -1947,11 +1932,10 @@ __device__ __forceinline__ PoolNodeCtx<C> load_pool_ctx(const PoolDomain<C> *p)
     return c;
 }
 
-// one node of a pool domain: its slots, the K17 collision and the ET scatter
-template <class S, bool EXACT, bool EVEN>
-__device__ __forceinline__ void pool_collide_node(S *base, const PoolNodeCtx<typename Codec<S>::compute> &dm, uint32_t k)
+// the slot nodes of node k of a pool domain
+template <class C>
+__device__ __forceinline__ void pool_slots(const PoolNodeCtx<C> &dm, uint32_t k, uint32_t (&nodes)[8])
 {
-    using C = typename Codec<S>::compute;
     const int nx = dm.nx, ny = dm.ny, nz = dm.nz, flags = dm.flags;
     const uint32_t yz = fast_div(k, dm.div_nx), x = k - yz * (uint32_t)nx;
     const uint32_t z = fast_div(yz, dm.div_ny), y = yz - z * (uint32_t)ny;
@@ -1961,7 +1945,6 @@ __device__ __forceinline__ void pool_collide_node(S *base, const PoolNodeCtx<typ
     const uint32_t sx = (uint32_t)(xp - (int)x);
     const uint32_t sy = (uint32_t)((yp - (int)y) * nx);
     const uint32_t sz = (uint32_t)((int64_t)(zp - (int)z) * nx * ny);
-    uint32_t nodes[8];
     nodes[0] = k;
     nodes[1] = k + sx;
     nodes[2] = k + sy;
@@ -1970,30 +1953,72 @@ __device__ __forceinline__ void pool_collide_node(S *base, const PoolNodeCtx<typ
     nodes[5] = k + sx + sz;
     nodes[6] = k + sy + sz;
     nodes[7] = k + sx + sy + sz;
-    C f[27];
-    gather_pre<S, EVEN>(base, dm.pitch, nodes, f);
-    C drho, vx, vy, vz;
-    collide<C, EXACT>(f, dm.rates, dm.fx, dm.fy, dm.fz, drho, vx, vy, vz);
-    scatter_post<S, EVEN>(base, dm.pitch, nodes, f);
 }
 
-// The pool's collision: a persistent grid over {domain, first node} items of blockDim x
-// nodes_per_thread nodes. Warp w of a block owns the 32-node segments it.y + w 32 + j blockDim.
-// By default every lane collides its node of each segment, skipping solid nodes. In a domain
-// flagged kPoolCompact (porous media, where most segments mix fluid and solid nodes) the warp
-// queues the fluid nodes of its segments in shared memory (a ballot per segment, in node order)
-// and collides them 32 at a time, so lanes are not left idle on solid nodes. Each node's arithmetic
-// is the same either way.
-// two resident blocks of 256 threads (or four of 128) for the FP32-arithmetic forms: at most 128
-// registers, the budget every FP32 collision fits without spills; FP64 takes what it needs
+// nodes a thread collides together: two in packed FP32x2 arithmetic (the FP32-arithmetic forms), else
+// one. NARROW: every domain's planes stay below 4 GB (slot_at)
+template <class S, bool EXACT, bool NARROW>
+constexpr int pool_width() { return sizeof(typename Codec<S>::compute) == 4 && !EXACT && NARROW ? 2 : 1; }
+
+// the slots, the K17 collision and the ET scatter of a thread's nodes of a pool domain
+template <class S, bool EXACT, bool EVEN, bool NARROW, int W>
+__device__ __forceinline__ void pool_collide_nodes(S *base, const PoolNodeCtx<typename Codec<S>::compute> &dm,
+                                                   const uint32_t (&k)[W], const bool (&act)[W])
+{
+    using C = typename Codec<S>::compute;
+    if constexpr (W == 1) {
+        if (!act[0])
+            return;
+        uint32_t nodes[8];
+        pool_slots(dm, k[0], nodes);
+        C f[27];
+        gather_pre<S, EVEN, NARROW>(base, dm.pitch, nodes, f);
+        C drho, vx, vy, vz;
+        collide<C, EXACT>(f, dm.rates, dm.fx, dm.fy, dm.fz, drho, vx, vy, vz);
+        scatter_post<S, EVEN, NARROW>(base, dm.pitch, nodes, f);
+    } else {
+        if (!act[0] && !act[1])
+            return;
+        uint32_t na[8], nb[8];
+        pool_slots(dm, k[0], na);
+        pool_slots(dm, k[1], nb);
+        // an inactive partner collides a rest state: finite, never stored
+        float fa[27], fb[27], ma[4], mb[4];
+        if (act[0]) gather_pre<S, EVEN, NARROW>(base, dm.pitch, na, fa);
+        else
+#pragma unroll
+            for (int d = 0; d < 27; ++d) fa[d] = 0.f;
+        if (act[1]) gather_pre<S, EVEN, NARROW>(base, dm.pitch, nb, fb);
+        else
+#pragma unroll
+            for (int d = 0; d < 27; ++d) fb[d] = 0.f;
+        collide_pair(fa, fb, dm.rates, dm.fx, dm.fy, dm.fz, ma, mb);
+        if (act[0])
+            scatter_post<S, EVEN, NARROW>(base, dm.pitch, na, fa);
+        if (act[1])
+            scatter_post<S, EVEN, NARROW>(base, dm.pitch, nb, fb);
+    }
+}
+
+// The pool's collision over {domain, first node} items of blockDim x nodes_per_thread nodes (one block
+// per item, or a persistent grid). A thread collides W nodes 32 apart, so a warp takes 32 W
+// consecutive nodes at a time: warp w of a block those from it.y + w 32 W in steps of blockDim W.
+// By default every lane collides its nodes, skipping solid ones. In a domain flagged kPoolCompact
+// (porous media, where most segments mix fluid and solid nodes) the warp queues the fluid nodes of
+// its segments in shared memory (a ballot per segment, in node order) and collides them 32 W at a
+// time, so lanes are not left idle on solid nodes. Each node's arithmetic is the same either way.
+// The FP32-arithmetic forms are held to 128 registers, two blocks of 256 threads or four of 128: with
+// 157-168 registers and three blocks of 128 the two-node kernel took 37.6 ms for 48 FP16 steps of
+// 192 ducts, with four 32.9 ms, and one node per thread 36.1 ms. FP64 takes what it needs.
 template <class S>
 constexpr int pool_min_blocks() { return sizeof(typename Codec<S>::compute) == 8 ? 1 : 2; }
 
-template <class S, bool EXACT, bool EVEN>
+template <class S, bool EXACT, bool EVEN, bool NARROW>
 __global__ void __launch_bounds__(256, pool_min_blocks<S>()) k17_pool_kernel(PoolArgs<typename Codec<S>::compute> a)
 {
     using C = typename Codec<S>::compute;
-    __shared__ uint32_t queue[8][64];
+    constexpr int W = pool_width<S, EXACT, NARROW>();
+    __shared__ uint32_t queue[8][32 * (W + 1)];
     __shared__ PoolNodeCtx<C> ctx;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lanes_below = (1u << lane) - 1u;
@@ -2012,38 +2037,54 @@ __global__ void __launch_bounds__(256, pool_min_blocks<S>()) k17_pool_kernel(Poo
         const uint32_t end = min(it.y + span, nodes_total);
         const uint8_t *mask =
             (dm.flags & kPoolMask) ? static_cast<const uint8_t *>(a.arena) + __ldg(&dp->mask_offset) : nullptr;
-        if (!(dm.flags & kPoolCompact)) {
-#pragma unroll 1
-            for (uint32_t k = it.y + threadIdx.x; k < end; k += blockDim.x) {
-                if (mask && __ldg(mask + k) == 0)
-                    continue;
-                pool_collide_node<S, EXACT, EVEN>(base, dm, k);
-            }
-            continue;
-        }
+        const bool compact = dm.flags & kPoolCompact;
         uint32_t *q = queue[warp];
         uint32_t pending = 0;            // queued fluid nodes (the same in every lane)
+        // a warp's next segment: the W segments of a step are neighbours
+        uint32_t seg = it.y + 32u * W * warp, part = 0;
 #pragma unroll 1
-        for (uint32_t seg = it.y + 32u * warp; seg < end; seg += blockDim.x) {
-            const uint32_t k = seg + lane;
-            const bool fluid = k < end && __ldg(mask + k) != 0;
-            const uint32_t ballot = __ballot_sync(0xffffffffu, fluid);
-            if (fluid)
-                q[pending + __popc(ballot & lanes_below)] = k;
-            pending += __popc(ballot);
-            __syncwarp();
-            if (pending >= 32u) {
-                pool_collide_node<S, EXACT, EVEN>(base, dm, q[lane]);
-                pending -= 32u;
-                const uint32_t rest = lane < pending ? q[32u + lane] : 0u;
+        for (;;) {
+            uint32_t k[W];
+            bool act[W];
+            if (!compact) {
+                if (seg >= end)
+                    break;
+#pragma unroll
+                for (int p = 0; p < W; ++p) {
+                    k[p] = seg + 32u * p + lane;
+                    act[p] = k[p] < end && (!mask || __ldg(mask + k[p]) != 0);
+                }
+                seg += blockDim.x * W;
+            } else {
+                while (pending < 32u * W && seg < end) {
+                    const uint32_t kk = seg + 32u * part + lane;
+                    const bool fluid = kk < end && __ldg(mask + kk) != 0;
+                    const uint32_t ballot = __ballot_sync(0xffffffffu, fluid);
+                    if (fluid)
+                        q[pending + __popc(ballot & lanes_below)] = kk;
+                    pending += __popc(ballot);
+                    if (++part == W) {
+                        part = 0;
+                        seg += blockDim.x * W;
+                    }
+                }
+                if (!pending)
+                    break;
                 __syncwarp();
-                if (lane < pending)
+#pragma unroll
+                for (int p = 0; p < W; ++p) {
+                    act[p] = 32u * p + lane < pending;
+                    k[p] = act[p] ? q[32u * p + lane] : 0u;
+                }
+                const uint32_t left = pending > 32u * W ? pending - 32u * W : 0u;   // < 32
+                const uint32_t rest = lane < left ? q[32u * W + lane] : 0u;
+                __syncwarp();
+                if (lane < left)
                     q[lane] = rest;
-                __syncwarp();
+                pending = left;
             }
+            pool_collide_nodes<S, EXACT, EVEN, NARROW, W>(base, dm, k, act);
         }
-        if (lane < pending)
-            pool_collide_node<S, EXACT, EVEN>(base, dm, q[lane]);
         __syncwarp();
     }
 }

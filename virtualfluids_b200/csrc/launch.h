@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "addr.h"
@@ -51,12 +52,19 @@ inline int box_block_x(int nx)
     int b = ((nx + 31) / 32) * 32;
     return b > 128 ? 128 : b;
 }
-// upper bound of the per-step energy partials any box kernel writes (one per warp of the direct
-// kernel's grid; the persistent kernels write fewer)
+// threads per block of the kernels that take the nodes in order: 128, or less where a small box
+// would leave SMs without a block
+inline unsigned box_threads(uint64_t n)
+{
+    return n >= 148ull * 128 * 2 ? 128u : n >= 148ull * 64 * 2 ? 64u : 32u;
+}
+// upper bound of the per-step energy partials any box kernel writes (one per warp of its grid;
+// the persistent kernels write fewer)
 inline uint64_t box_blocks(const BoxState &b)
 {
     const int bx = box_block_x(b.nx);
-    return (uint64_t)((b.nx + bx - 1) / bx) * (uint64_t)b.ny * (uint64_t)b.nz * (uint64_t)(bx / 32);
+    const uint64_t n = (uint64_t)b.nx * (uint64_t)b.ny * (uint64_t)b.nz;
+    return std::max((uint64_t)((b.nx + bx - 1) / bx) * (uint64_t)b.ny * (uint64_t)b.nz * (uint64_t)(bx / 32), n / 32 + 4);
 }
 
 // a pool domain's record as the host describes it (offsets in bytes from the arena start, except
@@ -101,9 +109,9 @@ struct PoolDomainSpec {
         static cudaError_t box_macros(const BoxState &b, bool even, void *rho, void *ux, void *uy, void *uz,       \
                                       cudaStream_t s);                                                             \
         static cudaError_t pool_collide(void *arena, const void *domains, const uint2 *items,                      \
-                                        const uint32_t *n_items, int nodes_per_thread, bool even, unsigned grid,   \
-                                        unsigned block, cudaStream_t s);                                           \
-        static const void *pool_kernel(bool even);                                                                \
+                                        const uint32_t *n_items, int nodes_per_thread, bool even, bool narrow,     \
+                                        unsigned grid, unsigned block, cudaStream_t s);                            \
+        static const void *pool_kernel(bool even, bool narrow);                                                    \
         static size_t pool_domain_bytes();                                                                        \
         static void pool_domain(void *out, const PoolDomainSpec &spec);                                            \
         static cudaError_t pool_mass(void *arena, const void *domains, const uint2 *items, uint32_t n_items,       \

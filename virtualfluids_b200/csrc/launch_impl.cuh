@@ -246,7 +246,8 @@ cudaError_t Launchers<S>::pressure(const vfb_level *L, const vfb_directional_bc 
 
 template <class S>
 cudaError_t Launchers<S>::pool_collide(void *arena, const void *domains, const uint2 *items, const uint32_t *n_items,
-                                       int nodes_per_thread, bool even, unsigned grid, unsigned block, cudaStream_t s)
+                                       int nodes_per_thread, bool even, bool narrow, unsigned grid, unsigned block,
+                                       cudaStream_t s)
 {
     using C = typename Codec<S>::compute;
     PoolArgs<C> a;
@@ -255,16 +256,27 @@ cudaError_t Launchers<S>::pool_collide(void *arena, const void *domains, const u
     a.items = items;
     a.n_items = n_items;
     a.nodes_per_thread = nodes_per_thread;
-    if (even) k17_pool_kernel<S, VFB_EXACT, true><<<grid, block, 0, s>>>(a);
-    else k17_pool_kernel<S, VFB_EXACT, false><<<grid, block, 0, s>>>(a);
+    if constexpr (sizeof(S) <= 4) {
+        if (narrow) {
+            if (even) k17_pool_kernel<S, VFB_EXACT, true, true><<<grid, block, 0, s>>>(a);
+            else k17_pool_kernel<S, VFB_EXACT, false, true><<<grid, block, 0, s>>>(a);
+            return cudaGetLastError();
+        }
+    }
+    if (even) k17_pool_kernel<S, VFB_EXACT, true, false><<<grid, block, 0, s>>>(a);
+    else k17_pool_kernel<S, VFB_EXACT, false, false><<<grid, block, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 template <class S>
-const void *Launchers<S>::pool_kernel(bool even)
+const void *Launchers<S>::pool_kernel(bool even, bool narrow)
 {
-    return even ? reinterpret_cast<const void *>(k17_pool_kernel<S, VFB_EXACT, true>)
-                : reinterpret_cast<const void *>(k17_pool_kernel<S, VFB_EXACT, false>);
+    if constexpr (sizeof(S) <= 4)
+        if (narrow)
+            return even ? reinterpret_cast<const void *>(k17_pool_kernel<S, VFB_EXACT, true, true>)
+                        : reinterpret_cast<const void *>(k17_pool_kernel<S, VFB_EXACT, false, true>);
+    return even ? reinterpret_cast<const void *>(k17_pool_kernel<S, VFB_EXACT, true, false>)
+                : reinterpret_cast<const void *>(k17_pool_kernel<S, VFB_EXACT, false, false>);
 }
 
 template <class S>
@@ -544,7 +556,11 @@ BoxCollideArgs<C> box_args(const BoxState &b)
     a.fz = (C)b.fz;
     a.energy_partials = nullptr;
     a.rho = a.vx = a.vy = a.vz = nullptr;
-    a.z_begin = 0;
+    a.first = 0;
+    a.count = (uint32_t)((uint64_t)b.nx * b.ny * b.nz);
+    a.exact_div = b.nx < (1 << 16) && b.ny < (1 << 16) && (uint64_t)b.nx * b.ny * b.nz < (1ull << 31);
+    a.div_nx = make_fast_div((uint32_t)b.nx);
+    a.div_ny = make_fast_div((uint32_t)b.ny);
     return a;
 }
 inline dim3 box_grid(const BoxState &b)
@@ -684,6 +700,36 @@ cudaError_t launch_box_pipe(const BoxCollideArgs<typename Codec<S>::compute> &a,
         *n_partials = (uint64_t)grid * (uint64_t)(B / 32);
     return cudaGetLastError();
 }
+// one node per thread; FP64 takes 64-bit slot addresses (its registers allow them)
+template <class S>
+void launch_box_direct(const BoxCollideArgs<typename Codec<S>::compute> &a, bool even, bool narrow, unsigned G, unsigned B,
+                       cudaStream_t s)
+{
+    const bool mask = a.mask != nullptr, energy = a.energy_partials != nullptr;
+    auto launch = [&](auto narrow_planes_c) {
+        constexpr bool W = decltype(narrow_planes_c)::value;
+#define VFB_K17B(E, M, N) k17_box_kernel<S, VFB_EXACT, E, M, N, W><<<G, B, 0, s>>>(a)
+        if (even) {
+            if (mask && energy) VFB_K17B(true, true, true);
+            else if (mask) VFB_K17B(true, true, false);
+            else if (energy) VFB_K17B(true, false, true);
+            else VFB_K17B(true, false, false);
+        } else {
+            if (mask && energy) VFB_K17B(false, true, true);
+            else if (mask) VFB_K17B(false, true, false);
+            else if (energy) VFB_K17B(false, false, true);
+            else VFB_K17B(false, false, false);
+        }
+#undef VFB_K17B
+    };
+    if constexpr (sizeof(S) <= 4) {
+        if (narrow) {
+            launch(std::true_type{});
+            return;
+        }
+    }
+    launch(std::false_type{});
+}
 } // namespace
 
 template <class S>
@@ -726,12 +772,13 @@ cudaError_t Launchers<S>::box_collide(const BoxState &b, bool even, double *part
 #undef VFB_K17Q
     }
     if constexpr (std::is_same<C, float>::value && !VFB_EXACT) {
-        if (b.variant == 4) {
-            // two rows per block row of the grid, packed FP32x2 arithmetic
-            const int bx = box_block_x(b.nx);
-            const dim3 G((unsigned)((b.nx + bx - 1) / bx), (unsigned)((b.ny + 1) / 2), (unsigned)b.nz), B(bx);
+        // two nodes per thread where they fill the device: 148 SMs x 4 blocks x 256 nodes. Below
+        // that one node per thread spreads the box over more warps (32^3 in FP32: 4.1 against 6.2 us
+        // per step; 64^3: equal)
+        if (narrow_planes(b.pitch, sizeof(S)) && (b.variant == 4 || (b.variant == 0 && a.count >= 148u * 4u * 256u))) {
+            const unsigned B = box_threads(a.count / 2), G = grid1d(((uint64_t)a.count + 1) / 2, B);
             if (n_partials)
-                *n_partials = (uint64_t)G.x * G.y * G.z * (B.x / 32);
+                *n_partials = (uint64_t)G * (B / 32);
 #define VFB_K17P(E, M, N) k17_box_pair_kernel<S, E, M, N><<<G, B, 0, s>>>(a)
             if (even) {
                 if (mask && energy) VFB_K17P(true, true, true);
@@ -764,22 +811,10 @@ cudaError_t Launchers<S>::box_collide(const BoxState &b, bool even, double *part
         }
 #undef VFB_K17T
     }
-    const dim3 G = box_grid(b), B(box_block_x(b.nx));
+    const unsigned B = box_threads(a.count), G = grid1d(a.count, B);
     if (n_partials)
-        *n_partials = (uint64_t)G.x * G.y * G.z * (B.x / 32);
-#define VFB_K17B(E, M, N) k17_box_kernel<S, VFB_EXACT, E, M, N, false><<<G, B, 0, s>>>(a)
-    if (even) {
-        if (mask && energy) VFB_K17B(true, true, true);
-        else if (mask) VFB_K17B(true, true, false);
-        else if (energy) VFB_K17B(true, false, true);
-        else VFB_K17B(true, false, false);
-    } else {
-        if (mask && energy) VFB_K17B(false, true, true);
-        else if (mask) VFB_K17B(false, true, false);
-        else if (energy) VFB_K17B(false, false, true);
-        else VFB_K17B(false, false, false);
-    }
-#undef VFB_K17B
+        *n_partials = (uint64_t)G * (B / 32);
+    launch_box_direct<S>(a, even, narrow_planes(b.pitch, sizeof(S)), G, B, s);
     return cudaGetLastError();
 }
 
@@ -810,18 +845,10 @@ cudaError_t Launchers<S>::box_collide_planes(const BoxState &b, bool even, int z
     if (z1 <= z0)
         return cudaSuccess;
     BoxCollideArgs<C> a = box_args<C>(b);
-    a.z_begin = z0;
-    dim3 G = box_grid(b);
-    G.z = (unsigned)(z1 - z0);
-    const dim3 B(box_block_x(b.nx));
-    const bool mask = b.mask != nullptr;
-    if (even) {
-        if (mask) k17_box_kernel<S, VFB_EXACT, true, true, false, false><<<G, B, 0, s>>>(a);
-        else k17_box_kernel<S, VFB_EXACT, true, false, false, false><<<G, B, 0, s>>>(a);
-    } else {
-        if (mask) k17_box_kernel<S, VFB_EXACT, false, true, false, false><<<G, B, 0, s>>>(a);
-        else k17_box_kernel<S, VFB_EXACT, false, false, false, false><<<G, B, 0, s>>>(a);
-    }
+    a.first = (uint32_t)((uint64_t)b.nx * b.ny * z0);
+    a.count = (uint32_t)((uint64_t)b.nx * b.ny * (z1 - z0));
+    const unsigned B = box_threads(a.count), G = grid1d(a.count, B);
+    launch_box_direct<S>(a, even, narrow_planes(b.pitch, sizeof(S)), G, B, s);
     return cudaGetLastError();
 }
 

@@ -43,9 +43,9 @@ uint64_t align_up(uint64_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
 // the launchers of one (storage, arithmetic) variant
 struct PoolOps {
-    cudaError_t (*collide)(void *, const void *, const uint2 *, const uint32_t *, int, bool, unsigned, unsigned,
+    cudaError_t (*collide)(void *, const void *, const uint2 *, const uint32_t *, int, bool, bool, unsigned, unsigned,
                            cudaStream_t);
-    const void *(*kernel)(bool);
+    const void *(*kernel)(bool, bool);
     size_t (*domain_bytes)();
     void (*domain)(void *, const vfb::PoolDomainSpec &);
     cudaError_t (*bcs)(void *, const void *, const uint2 *, const uint32_t *, const uint2 *, const uint32_t *,
@@ -166,6 +166,7 @@ struct vfb_pool {
     uint32_t *n_items = nullptr;
     size_t items_capacity = 0;
     bool list_dirty = true;
+    bool narrow = true;                // every active domain's planes allow 32-bit slot offsets
     uint64_t active_nodes = 0;
     bool even = true;
     int threads = 128, nodes_per_thread = 8, blocks_per_sm = -1, use_graph = 1;  // the default launch shape
@@ -215,7 +216,7 @@ cudaError_t update_grid(vfb_pool *p)
     }
     int bps = p->blocks_per_sm;
     int occ = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p->ops.kernel(true), p->threads, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p->ops.kernel(true, p->narrow), p->threads, 0);
     if (e != cudaSuccess)
         return e;
     if (bps <= 0 || bps > occ)
@@ -308,15 +309,22 @@ cudaError_t rebuild_list(vfb_pool *p, cudaStream_t s)
     const uint64_t span = (uint64_t)p->threads * (uint64_t)p->nodes_per_thread;
     std::vector<uint2> items;
     uint64_t nodes = 0;
+    bool narrow = true;
     for (uint32_t id = 0; id < p->slots.size(); ++id) {
         const DomainSlot &d = p->slots[id];
         if (!d.live || !d.active)
             continue;
         nodes += d.nodes;
+        narrow = narrow && vfb::narrow_planes(d.pitch, storage_size(p->desc.storage));
         for (uint64_t l0 = 0; l0 < d.nodes; l0 += span)
             items.push_back(make_uint2(id, (unsigned)l0));
     }
     cudaError_t e = cudaSuccess;
+    if (narrow != p->narrow) {
+        drop_graph(p);                 // another kernel, with its own persistent grid
+        p->narrow = narrow;
+        e = update_grid(p);
+    }
     if (items.size() > p->items_capacity) {
         // a new buffer: a captured step refers to the old one
         drop_graph(p);
@@ -353,7 +361,7 @@ cudaError_t rebuild_list(vfb_pool *p, cudaStream_t s)
 cudaError_t launch_step(vfb_pool *p, bool even, cudaStream_t s)
 {
     ++p->launches;
-    cudaError_t e = p->ops.collide(p->arena, p->domain_table, p->items, p->n_items, p->nodes_per_thread, even, p->grid,
+    cudaError_t e = p->ops.collide(p->arena, p->domain_table, p->items, p->n_items, p->nodes_per_thread, even, p->narrow, p->grid,
                                    (unsigned)p->threads, s);
     if (e == cudaSuccess && (p->has_noslip || p->has_pressure)) {
         p->launches += (p->has_noslip ? 1 : 0) + (p->has_guard ? 1 : 0) + (p->has_pressure ? 1 : 0);

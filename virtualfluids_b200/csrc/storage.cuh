@@ -32,6 +32,24 @@ enum StorageKind : int { kStoreF64 = 0, kStoreF32 = 1, kStoreF16 = 2, kStoreBF16
 template <class S>
 struct Codec;
 
+// Node k's slot in a direction plane. NARROW (narrow_planes, addr.h): planes below 4 GB; the byte offset is a 32-bit product
+// added to the plane's pointer, which is the same for every thread. It needs one register per slot
+// class where 64-bit sums need two (the two-node FP32 kernel spilled 28-68 bytes with them at its
+// 128 registers, and took 671 instead of 589 us on 320 x 256 x 192).
+template <bool NARROW, class S>
+__device__ __forceinline__ S *slot_at(S *plane, uint32_t k)
+{
+    if constexpr (NARROW)
+        return reinterpret_cast<S *>(reinterpret_cast<char *>(plane) + k * (uint32_t)sizeof(S));
+    else
+        return plane + k;
+}
+template <bool NARROW, class S>
+__device__ __forceinline__ const S *slot_at(const S *plane, uint32_t k)
+{
+    return slot_at<NARROW>(const_cast<S *>(plane), k);
+}
+
 // float(1 / w_d) for a run-time d: the constants the 16-bit stores scale by
 __device__ __forceinline__ float inv_weight_rt(int d)
 {
@@ -67,11 +85,18 @@ struct Codec<float> {
 // value's bits and the slot's offset in its population array, so a run stays reproducible bit for
 // bit (the same domain computes the same bits wherever its array lives), and they change whenever
 // the value does. The conversion is sm_100a's cvt.rs (operand a lands in the upper half).
-__device__ __forceinline__ uint32_t sr_bits(float v, uint64_t off)
+__device__ __forceinline__ uint32_t sr_bits(float v, uint32_t off)
 {
-    // two odd multipliers carry the value's (noisy) low mantissa bits and the slot offset into
-    // every bit position; cheap, because the 16-bit forms are bound by arithmetic
-    return (__float_as_uint(v) * 0x9E3779B1u) ^ ((uint32_t)off * 0x85EBCA77u) ^ (uint32_t)(off >> 32);
+    // two odd multipliers carry the value's (noisy) low mantissa bits and the slot offset (its low 32
+    // bits) into every bit position; sums of products, because the 16-bit forms are bound by the
+    // instructions they issue: with off = plane + node, each product with the rest of the sum is
+    // one multiply-add
+    return __float_as_uint(v) * 0x9E3779B1u + off * 0x85EBCA77u;
+}
+// the bits of two values rounded together: the first one's, moved by the second value
+__device__ __forceinline__ uint32_t sr_bits(float v0, float v1, uint32_t off0)
+{
+    return __float_as_uint(v1) * 0xC2B2AE35u + sr_bits(v0, off0);
 }
 
 __device__ __forceinline__ __half half_sr(float v, uint32_t rbits)
@@ -107,13 +132,15 @@ template <>
 struct Codec<__half> {
     using compute = float;
     static constexpr bool kPairs = true;
-    __device__ __forceinline__ static void store_pair_at(__half *base, uint64_t off0, float v0, int d0, uint64_t off1,
-                                                         float v1, int d1)
+    // two slots, node k of the plane at p each; off0: slot p0's plane in its array (low 32 bits)
+    template <bool NARROW>
+    __device__ __forceinline__ static void store_pair(__half *p0, uint32_t k0, uint32_t off0, float v0, int d0, __half *p1,
+                                                      uint32_t k1, float v1, int d1)
     {
         const float s0 = v0 * float(1.0 / weight(d0)), s1 = v1 * float(1.0 / weight(d1));
-        const uint32_t h = half2_sr(s0, s1, sr_bits(s0, off0) ^ (__float_as_uint(s1) * 0xC2B2AE35u));
-        base[off0] = __ushort_as_half((unsigned short)(h >> 16));
-        base[off1] = __ushort_as_half((unsigned short)(h & 0xffffu));
+        const uint32_t h = half2_sr(s0, s1, sr_bits(s0, s1, off0 + k0));
+        *slot_at<NARROW>(p0, k0) = __ushort_as_half((unsigned short)(h >> 16));
+        *slot_at<NARROW>(p1, k1) = __ushort_as_half((unsigned short)(h & 0xffffu));
     }
     // the decoding product is rounded on its own (never fused into a later addition), so a decoded
     // value is the same float wherever it is used or saved
@@ -121,13 +148,13 @@ struct Codec<__half> {
     __device__ __forceinline__ static void store_at(__half *base, uint64_t off, float v, int d)
     {
         const float s = v * float(1.0 / weight(d));
-        base[off] = half_sr(s, sr_bits(s, off));
+        base[off] = half_sr(s, sr_bits(s, (uint32_t)off));
     }
     // store_at for a direction known only at run time (the same scale factors)
     __device__ __forceinline__ static void store_at_rt(__half *base, uint64_t off, float v, int d)
     {
         const float s = v * inv_weight_rt(d);
-        base[off] = half_sr(s, sr_bits(s, off));
+        base[off] = half_sr(s, sr_bits(s, (uint32_t)off));
     }
 };
 
@@ -135,13 +162,15 @@ template <>
 struct Codec<__nv_bfloat16> {
     using compute = float;
     static constexpr bool kPairs = true;
-    __device__ __forceinline__ static void store_pair_at(__nv_bfloat16 *base, uint64_t off0, float v0, int d0,
-                                                         uint64_t off1, float v1, int d1)
+    // two slots, node k of the plane at p each; off0: slot p0's plane in its array (low 32 bits)
+    template <bool NARROW>
+    __device__ __forceinline__ static void store_pair(__nv_bfloat16 *p0, uint32_t k0, uint32_t off0, float v0, int d0, __nv_bfloat16 *p1,
+                                                      uint32_t k1, float v1, int d1)
     {
         const float s0 = v0 * float(1.0 / weight(d0)), s1 = v1 * float(1.0 / weight(d1));
-        const uint32_t h = bf162_sr(s0, s1, sr_bits(s0, off0) ^ (__float_as_uint(s1) * 0xC2B2AE35u));
-        base[off0] = __ushort_as_bfloat16((unsigned short)(h >> 16));
-        base[off1] = __ushort_as_bfloat16((unsigned short)(h & 0xffffu));
+        const uint32_t h = bf162_sr(s0, s1, sr_bits(s0, s1, off0 + k0));
+        *slot_at<NARROW>(p0, k0) = __ushort_as_bfloat16((unsigned short)(h >> 16));
+        *slot_at<NARROW>(p1, k1) = __ushort_as_bfloat16((unsigned short)(h & 0xffffu));
     }
     __device__ __forceinline__ static float load(const __nv_bfloat16 *p, int d)
     {
@@ -150,12 +179,12 @@ struct Codec<__nv_bfloat16> {
     __device__ __forceinline__ static void store_at(__nv_bfloat16 *base, uint64_t off, float v, int d)
     {
         const float s = v * float(1.0 / weight(d));
-        base[off] = bf16_sr(s, sr_bits(s, off));
+        base[off] = bf16_sr(s, sr_bits(s, (uint32_t)off));
     }
     __device__ __forceinline__ static void store_at_rt(__nv_bfloat16 *base, uint64_t off, float v, int d)
     {
         const float s = v * inv_weight_rt(d);
-        base[off] = bf16_sr(s, sr_bits(s, off));
+        base[off] = bf16_sr(s, sr_bits(s, (uint32_t)off));
     }
 };
 
@@ -229,14 +258,15 @@ struct Codec<e3m12_t> {
     // float constants, folded into their one multiplication
     __device__ __forceinline__ static float enc_scale(int d) { return float(1.0 / weight(d)) * 0x1p-120f; }
     __device__ __forceinline__ static float dec_scale(int d) { return float(weight(d)) * 0x1p120f; }
-    __device__ __forceinline__ static void store_pair_at(e3m12_t *base, uint64_t off0, float v0, int d0, uint64_t off1,
-                                                         float v1, int d1)
+    template <bool NARROW>
+    __device__ __forceinline__ static void store_pair(e3m12_t *p0, uint32_t k0, uint32_t off0, float v0, int d0,
+                                                      e3m12_t *p1, uint32_t k1, float v1, int d1)
     {
         const float t0 = v0 * enc_scale(d0), t1 = v1 * enc_scale(d1);
         // 11 random bits each from the upper bits of the hash (they mix all of the value's bits)
-        const uint32_t r = sr_bits(t0, off0) ^ (__float_as_uint(t1) * 0xC2B2AE35u);
-        base[off0].bits = e3m12::encode_scaled(t0, r >> 21);
-        base[off1].bits = e3m12::encode_scaled(t1, (r >> 10) & 0x7ffu);
+        const uint32_t r = sr_bits(t0, t1, off0 + k0);
+        slot_at<NARROW>(p0, k0)->bits = e3m12::encode_scaled(t0, r >> 21);
+        slot_at<NARROW>(p1, k1)->bits = e3m12::encode_scaled(t1, (r >> 10) & 0x7ffu);
     }
     // rounded on its own, as for the other 16-bit forms
     __device__ __forceinline__ static float load(const e3m12_t *p, int d)
@@ -246,12 +276,12 @@ struct Codec<e3m12_t> {
     __device__ __forceinline__ static void store_at(e3m12_t *base, uint64_t off, float v, int d)
     {
         const float t = v * enc_scale(d);
-        base[off].bits = e3m12::encode_scaled(t, sr_bits(t, off) >> 21);
+        base[off].bits = e3m12::encode_scaled(t, sr_bits(t, (uint32_t)off) >> 21);
     }
     __device__ __forceinline__ static void store_at_rt(e3m12_t *base, uint64_t off, float v, int d)
     {
         const float t = v * (inv_weight_rt(d) * 0x1p-120f);
-        base[off].bits = e3m12::encode_scaled(t, sr_bits(t, off) >> 21);
+        base[off].bits = e3m12::encode_scaled(t, sr_bits(t, (uint32_t)off) >> 21);
     }
 };
 

@@ -114,6 +114,20 @@ struct PressureArgs {
 };
 
 // ---------------------------------------------------------------------------------------------
+// The kernels of a time step follow one another in a stream, each reading what the one before wrote.
+// They are launched with programmatic stream serialisation (launch_next): every block lets the
+// next kernel's blocks be placed as soon as all of its own are, and waits here, before its first
+// access, until the kernel before has finished and its writes are visible. So only the launch and
+// the placement of a kernel overlap the one before; a step of small kernels is bound by these.
+// A kernel that nothing overlaps (launched without the attribute) passes through.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void chain_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------------------------
 // addressing
 // ---------------------------------------------------------------------------------------------
 
@@ -228,6 +242,7 @@ __device__ __forceinline__ void gather_post(const S *base, uint64_t n, const uin
 template <class S, bool EXACT, bool EVEN, bool WRITE_MACRO, bool BODY_FORCE>
 __global__ void __launch_bounds__(128) k17_list_kernel(ListCollideArgs<typename Codec<S>::compute> a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n_idx)
@@ -411,6 +426,7 @@ __device__ __forceinline__ void store_energy_partial(double *partials, double m,
 template <class S, bool EXACT, bool EVEN, bool MASK, bool ENERGY, bool NARROW>
 __global__ void __launch_bounds__(128, box_min_blocks<S>()) k17_box_kernel(BoxCollideArgs<typename Codec<S>::compute> a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t k = a.first + (uint32_t)i;
@@ -607,6 +623,7 @@ __global__ void __launch_bounds__(128, pipe_min_blocks<S>()) k17_box_pipe_kernel
 template <class S, bool EVEN, bool MASK, bool ENERGY>
 __global__ void __launch_bounds__(128, 4) k17_box_pair_kernel(BoxCollideArgs<float> a)
 {
+    chain_begin();
     const uint64_t i0 = 2ull * ((uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) + (threadIdx.x & 31u);
     bool act[2];
     uint32_t nodes[2][8];
@@ -972,6 +989,7 @@ __device__ __forceinline__ void load_link_q(const C *__restrict__ q27, uint64_t 
 template <class S, bool EVEN, bool VELOCITY>
 __global__ void __launch_bounds__(128) bc_bounce_back_kernel(BCArgs a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nbc)
@@ -1187,6 +1205,7 @@ __device__ __forceinline__ void bc_interpolated_node(S *base, uint64_t n, const 
 template <class S, bool EVEN, bool VELOCITY, int FORM = kBCCompressible>
 __global__ void __launch_bounds__(128) bc_interpolated_kernel(BCArgs a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nbc)
@@ -1229,6 +1248,7 @@ __device__ __forceinline__ void save_guarded(const S *__restrict__ base, uint64_
 template <class S, bool EVEN>
 __global__ void __launch_bounds__(128) bc_guard_kernel(BCArgs a, typename Codec<S>::compute *saved)
 {
+    chain_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nbc)
         return;
@@ -1247,6 +1267,7 @@ __global__ void __launch_bounds__(128) bc_guard_kernel(BCArgs a, typename Codec<
 template <class S, bool EVEN>
 __global__ void __launch_bounds__(128) bc_snapshot_kernel(BCArgs a, typename Codec<S>::compute *snap)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nbc)
@@ -1307,6 +1328,7 @@ __device__ __forceinline__ void bc_pressure_neq_node(S *base, uint64_t n, const 
 template <class S, bool EVEN, bool INCOMP = false>
 __global__ void __launch_bounds__(128) bc_pressure_neq_kernel(PressureArgs a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nbc)
@@ -1329,6 +1351,7 @@ __global__ void __launch_bounds__(128) bc_pressure_neq_kernel(PressureArgs a)
 template <class S, bool EVEN, bool CORRECTION>
 __global__ void __launch_bounds__(128) bc_outflow_kernel(PressureArgs a, double correction)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.nbc)
@@ -1716,6 +1739,7 @@ __device__ __forceinline__ void cell_coefficients_of_group(const S *base, uint64
 template <class S, bool COARSE_EVEN>
 __global__ void __launch_bounds__(128) scale_cf_kernel(ScaleArgs a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint64_t cell = t >> 3;
@@ -1754,6 +1778,7 @@ __global__ void __launch_bounds__(128) scale_cf_kernel(ScaleArgs a)
 template <class S, bool COARSE_EVEN>
 __global__ void __launch_bounds__(128) scale_fc_kernel(ScaleArgs a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint64_t cell = t >> 3;
@@ -2016,6 +2041,7 @@ constexpr int pool_min_blocks() { return sizeof(typename Codec<S>::compute) == 8
 template <class S, bool EXACT, bool EVEN, bool NARROW>
 __global__ void __launch_bounds__(256, pool_min_blocks<S>()) k17_pool_kernel(PoolArgs<typename Codec<S>::compute> a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     constexpr int W = pool_width<S, EXACT, NARROW>();
     __shared__ uint32_t queue[8][32 * (W + 1)];
@@ -2150,6 +2176,7 @@ struct PoolBCArgs {
 template <class S, bool EVEN>
 __global__ void __launch_bounds__(128) pool_noslip_guard_kernel(PoolBCArgs<typename Codec<S>::compute> a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t n_items = __ldg(a.n_items);
     for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x) {
@@ -2196,6 +2223,7 @@ template <class S, bool EVEN>
 __global__ void __launch_bounds__(128, sizeof(S) == 8 ? 4 : (sizeof(S) == 4 ? 8 : 7))
     pool_noslip_kernel(PoolBCArgs<typename Codec<S>::compute> a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     __shared__ LinkTile<C> tiles[kLinkWarps];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -2284,6 +2312,7 @@ __global__ void __launch_bounds__(128, sizeof(S) == 8 ? 4 : (sizeof(S) == 4 ? 8 
 template <class S, bool EVEN>
 __global__ void __launch_bounds__(128) pool_pressure_kernel(PoolBCArgs<typename Codec<S>::compute> a)
 {
+    chain_begin();
     using C = typename Codec<S>::compute;
     const uint32_t n_items = __ldg(a.n_items);
     for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x) {

@@ -2002,8 +2002,10 @@ int vfb_box_init(vfb_box *box, const void *rho, const void *ux, const void *uy, 
             dev[i] = f[i];
         }
     }
-    // PreProcessorImp::init (PreProcessorImp.cpp:50-58): odd parity, then even
-    if (e == cudaSuccess)
+    // PreProcessorImp::init (PreProcessorImp.cpp:50-58): odd parity, then even. In a periodic box without
+    // a mask every slot of every plane belongs to one node in either parity, so the even pass
+    // writes all that the odd one would
+    if (e == cudaSuccess && !vfb::every_slot_owned(box->state))
         e = VFB_DISPATCH(box->desc.storage, box->desc.arith, LA::box_init(box->state, false, dev[0], dev[1], dev[2], dev[3], s));
     if (e == cudaSuccess)
         e = VFB_DISPATCH(box->desc.storage, box->desc.arith, LA::box_init(box->state, true, dev[0], dev[1], dev[2], dev[3], s));

@@ -1525,18 +1525,12 @@ __global__ void __launch_bounds__(128) init_box_kernel(BoxCollideArgs<typename C
                                                        const void *ux, const void *uy, const void *uz)
 {
     using C = typename Codec<S>::compute;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y, z = blockIdx.z;
-    if (x >= a.nx)
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t k = a.first + (uint32_t)i;
+    if (i >= a.count || (a.mask && a.mask[k] == 0))
         return;
-    const uint32_t k = (uint32_t)((uint64_t)a.nx * ((uint64_t)y + (uint64_t)a.ny * z) + x);
-    if (a.mask && a.mask[k] == 0)
-        return;
-    const int xp = (x + 1 < a.nx) ? x + 1 : (a.periodic_x ? 0 : x);
-    const int yp = (y + 1 < a.ny) ? y + 1 : (a.periodic_y ? 0 : y);
-    const int zp = (z + 1 < a.nz) ? z + 1 : (a.periodic_z ? 0 : z);
-    const uint32_t sx = (uint32_t)(xp - x), sy = (uint32_t)((yp - y) * a.nx), sz = (uint32_t)((int64_t)(zp - z) * a.nx * a.ny);
-    const uint32_t nodes[8] = { k, k + sx, k + sy, k + sx + sy, k + sz, k + sx + sz, k + sy + sz, k + sx + sy + sz };
+    uint32_t nodes[8];
+    box_slots(a, k, nodes);
     const C drho = static_cast<const C *>(rho)[k];
     const C vx = static_cast<const C *>(ux)[k], vy = static_cast<const C *>(uy)[k], vz = static_cast<const C *>(uz)[k];
     const C cu_sq = C(1.5) * (vx * vx + vy * vy + vz * vz);
@@ -1598,11 +1592,10 @@ template <class S, bool EVEN>
 __global__ void __launch_bounds__(128) macros_box_kernel(BoxCollideArgs<typename Codec<S>::compute> a)
 {
     using C = typename Codec<S>::compute;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y, z = blockIdx.z;
-    if (x >= a.nx)
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t k = a.first + (uint32_t)i;
+    if (i >= a.count)
         return;
-    const uint32_t k = (uint32_t)((uint64_t)a.nx * ((uint64_t)y + (uint64_t)a.ny * z) + x);
     if (a.mask && a.mask[k] == 0) {
         a.rho[k] = C(0);
         a.vx[k] = C(0);
@@ -1610,11 +1603,8 @@ __global__ void __launch_bounds__(128) macros_box_kernel(BoxCollideArgs<typename
         a.vz[k] = C(0);
         return;
     }
-    const int xp = (x + 1 < a.nx) ? x + 1 : (a.periodic_x ? 0 : x);
-    const int yp = (y + 1 < a.ny) ? y + 1 : (a.periodic_y ? 0 : y);
-    const int zp = (z + 1 < a.nz) ? z + 1 : (a.periodic_z ? 0 : z);
-    const uint32_t sx = (uint32_t)(xp - x), sy = (uint32_t)((yp - y) * a.nx), sz = (uint32_t)((int64_t)(zp - z) * a.nx * a.ny);
-    const uint32_t nodes[8] = { k, k + sx, k + sy, k + sx + sy, k + sz, k + sx + sz, k + sy + sz, k + sx + sy + sz };
+    uint32_t nodes[8];
+    box_slots(a, k, nodes);
     C f[27];
     gather_pre<S, EVEN>(static_cast<const S *>(a.dist), a.pitch, nodes, f);
     const C r = density_pyramid(f);

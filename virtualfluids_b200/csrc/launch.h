@@ -46,6 +46,9 @@ struct BoxState {
     int *status;                  // device status word (DeviceError), nullable
 };
 
+// whether the nodes' slots of one parity are all slots of the array (a periodic box, every node fluid)
+inline bool every_slot_owned(const BoxState &b) { return b.periodic_x && b.periodic_y && b.periodic_z && !b.mask; }
+
 // block shape of the box kernels: x extent of a block (multiple of 32, at most 128)
 inline int box_block_x(int nx)
 {

@@ -900,7 +900,7 @@ cudaError_t Launchers<S>::box_init(const BoxState &b, bool even, const void *rho
 {
     using C = typename Codec<S>::compute;
     BoxCollideArgs<C> a = box_args<C>(b);
-    const dim3 G = box_grid(b), B(box_block_x(b.nx));
+    const unsigned B = box_threads(a.count), G = grid1d(a.count, B);
     if (even) init_box_kernel<S, true><<<G, B, 0, s>>>(a, rho, ux, uy, uz);
     else init_box_kernel<S, false><<<G, B, 0, s>>>(a, rho, ux, uy, uz);
     return cudaGetLastError();
@@ -915,7 +915,7 @@ cudaError_t Launchers<S>::box_macros(const BoxState &b, bool even, void *rho, vo
     a.vx = static_cast<C *>(ux);
     a.vy = static_cast<C *>(uy);
     a.vz = static_cast<C *>(uz);
-    const dim3 G = box_grid(b), B(box_block_x(b.nx));
+    const unsigned B = box_threads(a.count), G = grid1d(a.count, B);
     if (even) macros_box_kernel<S, true><<<G, B, 0, s>>>(a);
     else macros_box_kernel<S, false><<<G, B, 0, s>>>(a);
     return cudaGetLastError();

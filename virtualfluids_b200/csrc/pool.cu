@@ -846,7 +846,7 @@ int vfb_pool_init_domain(vfb_pool *p, uint32_t id, const void *rho, const void *
     // PreProcessorImp::init writes the odd, then the even parity; here the pool's current parity
     // is written last, so the domain joins the shared step sequence wherever it stands
     const vfb::BoxState b = domain_box(p, d);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && !vfb::every_slot_owned(b))
         e = p->ops.init(b, !p->even, dev[0], dev[1], dev[2], dev[3], s);
     if (e == cudaSuccess)
         e = p->ops.init(b, p->even, dev[0], dev[1], dev[2], dev[3], s);

@@ -8,6 +8,7 @@
 // weight, inverse) fold and the 27 populations stay in registers.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "addr.h"
 #include "interp.cuh"
@@ -45,12 +46,42 @@ __device__ __forceinline__ uint32_t checked_node(uint32_t v, uint64_t n)
 #define VFB_NODE(v, n) (v)
 #endif
 
+// Where the 27 direction planes start. In the kernels' parameters (PlaneTable) a plane's pointer is a
+// constant operand of the one multiply-add that forms a slot's address; formed from a base and a
+// stride, every slot costs two additions more (FP16, two nodes per thread: 1576 against 1456
+// instructions, FP32 1320 against 1184, and registers to spare). PlaneStride serves the kernels
+// that are bound by something else.
+struct PlaneTable {
+    void *p[27];
+    template <class S>
+    __device__ __forceinline__ S *slot(int i, uint32_t k) const { return static_cast<S *>(p[i]) + k; }
+};
+struct PlaneStride {
+    void *base;
+    uint64_t n;
+    template <class S>
+    __device__ __forceinline__ S *slot(int i, uint32_t k) const { return static_cast<S *>(base) + (uint64_t)i * n + k; }
+};
+// a stride whose planes stay below 4 GB (narrow_planes, addr.h): 32-bit byte offsets within a plane,
+// one register per slot class instead of two. For the pool, whose planes start elsewhere for every
+// work item: 48 FP16 steps of 192 ducts 32.2 ms, with 64-bit offsets 35.7, with the planes'
+// pointers in shared memory 33.2
+struct PlaneNarrow {
+    void *base;
+    uint64_t n;
+    template <class S>
+    __device__ __forceinline__ S *slot(int i, uint32_t k) const
+    {
+        return reinterpret_cast<S *>(reinterpret_cast<char *>(static_cast<S *>(base) + (uint64_t)i * n) + k * (uint32_t)sizeof(S));
+    }
+};
+
 // ---------------------------------------------------------------------------------------------
 // argument packs
 // ---------------------------------------------------------------------------------------------
 template <class C>
 struct ListCollideArgs {
-    void *dist;                 // distributions.f[0]
+    PlaneTable planes;          // distributions.f[0] ... f[26]
     uint64_t n;                 // numberOfNodes (plane stride)
     const uint32_t *nbx, *nby, *nbz;
     const uint32_t *idx;        // fluid node indices
@@ -69,6 +100,7 @@ template <class C>
 struct BoxCollideArgs {
     void *dist;                 // 27 planes of `pitch` elements, node k = x + nx (y + ny z)
     uint64_t pitch;
+    PlaneTable planes;          // their pointers
     int nx, ny, nz;
     int periodic_x, periodic_y, periodic_z;
     const uint8_t *mask;        // optional: nonzero = collide (fluid); nullptr = every node
@@ -197,32 +229,119 @@ __device__ __forceinline__ void node_slots(uint32_t k, const uint32_t *nbx, cons
         box_nodes(k, b, nodes);
 }
 
-template <class S, bool EVEN, bool NARROW = false>
-__device__ __forceinline__ void gather_pre(const S *__restrict__ base, uint64_t n, const uint32_t (&nodes)[8],
-                                           typename Codec<S>::compute (&f)[27])
+// FP64 with FMA arithmetic is bound by memory, and was 6 % slower with the table (256^3 1205 against
+// 1130 us per step); the exact form gains 0.8 % from it
+template <class S, bool EXACT>
+constexpr bool plane_table_pays() { return sizeof(typename Codec<S>::compute) == 4 || EXACT; }
+template <class S, bool EXACT>
+__device__ __forceinline__ auto planes_of(const PlaneTable &t, uint64_t n)
+{
+    if constexpr (plane_table_pays<S, EXACT>())
+        return t;
+    else
+        return PlaneStride{ t.p[0], n };
+}
+
+template <class S, bool EVEN, class P>
+__device__ __forceinline__ void gather_planes(const P &planes, const uint32_t (&nodes)[8], typename Codec<S>::compute (&f)[27])
 {
 #pragma unroll
     for (int d = 0; d < 27; ++d)
-        f[d] = Codec<S>::load(slot_at<NARROW>(base + (uint64_t)plane<EVEN>(d) * n, nodes[shift_class(d)]), d);
+        f[d] = Codec<S>::load(planes.template slot<S>(plane<EVEN>(d), nodes[shift_class(d)]), d);
+}
+template <class S, bool EVEN>
+__device__ __forceinline__ void gather_pre(const S *base, uint64_t n, const uint32_t (&nodes)[8],
+                                           typename Codec<S>::compute (&f)[27])
+{
+    gather_planes<S, EVEN>(PlaneStride{ const_cast<S *>(base), n }, nodes, f);
 }
 
-// setPostCollisionDistribution (KernelUtilities.h:350): the slot of d receives f[inv d]
-template <class S, bool EVEN, bool NARROW = false>
-__device__ __forceinline__ void scatter_post(S *__restrict__ base, uint64_t n, const uint32_t (&nodes)[8],
-                                             const typename Codec<S>::compute (&f)[27])
+// setPostCollisionDistribution (KernelUtilities.h:350): the slot of d receives f[inv d]. 16-bit
+// storage: f holds the scaled values (enc_scale), and two directions share one stochastic-rounding
+// conversion.
+template <class S, bool EVEN, class P>
+__device__ __forceinline__ void scatter_scaled(const P &planes, const uint32_t (&nodes)[8],
+                                               const typename Codec<S>::compute (&f)[27])
 {
     if constexpr (Codec<S>::kPairs) {
-        // 16-bit storage: two directions share one stochastic-rounding conversion
 #pragma unroll
         for (int d = 0; d + 1 < 27; d += 2)
-            Codec<S>::template store_pair<NARROW>(base + (uint64_t)plane<EVEN>(d) * n, nodes[shift_class(d)],
-                                 (uint32_t)((uint64_t)plane<EVEN>(d) * n), f[inv(d)], d,
-                                 base + (uint64_t)plane<EVEN>(d + 1) * n, nodes[shift_class(d + 1)], f[inv(d + 1)], d + 1);
-        Codec<S>::store_at(base, (uint64_t)plane<EVEN>(26) * n + nodes[shift_class(26)], f[inv(26)], 26);
+            Codec<S>::store_pair(planes.template slot<S>(plane<EVEN>(d), nodes[shift_class(d)]), nodes[shift_class(d)],
+                                 plane<EVEN>(d), f[inv(d)],
+                                 planes.template slot<S>(plane<EVEN>(d + 1), nodes[shift_class(d + 1)]), f[inv(d + 1)]);
+        Codec<S>::store_scaled(planes.template slot<S>(plane<EVEN>(26), nodes[shift_class(26)]), nodes[shift_class(26)],
+                               plane<EVEN>(26), f[inv(26)]);
     } else {
 #pragma unroll
         for (int d = 0; d < 27; ++d)
-            Codec<S>::store(slot_at<NARROW>(base + (uint64_t)plane<EVEN>(d) * n, nodes[shift_class(d)]), f[inv(d)], d);
+            Codec<S>::store(planes.template slot<S>(plane<EVEN>(d), nodes[shift_class(d)]), f[inv(d)], d);
+    }
+}
+template <class S, bool EVEN, class P>
+__device__ __forceinline__ void scatter_planes(const P &planes, const uint32_t (&nodes)[8],
+                                               const typename Codec<S>::compute (&f)[27])
+{
+    if constexpr (Codec<S>::kPairs) {
+        typename Codec<S>::compute g[27];
+#pragma unroll
+        for (int d = 0; d < 27; ++d)
+            g[d] = f[d] * Codec<S>::enc_scale(d);
+        scatter_scaled<S, EVEN>(planes, nodes, g);
+    } else {
+        scatter_scaled<S, EVEN>(planes, nodes, f);
+    }
+}
+template <class S, bool EVEN>
+__device__ __forceinline__ void scatter_post(S *base, uint64_t n, const uint32_t (&nodes)[8],
+                                             const typename Codec<S>::compute (&f)[27])
+{
+    scatter_planes<S, EVEN>(PlaneStride{ base, n }, nodes, f);
+}
+
+// the slots, the K17 collision and the ET scatter of two nodes in packed FP32x2 arithmetic; mac: drho and
+// velocity of each. An inactive partner collides a rest state (drho = 0, u = 0): finite, never
+// stored. The populations are decoded one by one: the compiler contracts a packed decoding product
+// with the sum it feeds, and the bits would differ from those of one node per thread.
+template <class S, bool EVEN, class P>
+__device__ __forceinline__ void collide_two(const P &planes, const uint32_t (&na)[8], const uint32_t (&nb)[8], bool a,
+                                            bool b, const K17Rates<float> &r, float fx, float fy, float fz,
+                                            float (&mac)[2][4])
+{
+    float fa[27], fb[27];
+    if (a) gather_planes<S, EVEN>(planes, na, fa);
+    else
+#pragma unroll
+        for (int d = 0; d < 27; ++d) fa[d] = 0.f;
+    if (b) gather_planes<S, EVEN>(planes, nb, fb);
+    else
+#pragma unroll
+        for (int d = 0; d < 27; ++d) fb[d] = 0.f;
+    f2 f[27], m[4];
+#pragma unroll
+    for (int d = 0; d < 27; ++d)
+        f[d] = f2(fa[d], fb[d]);
+    k17_collide_fast<f2, float>(f, r, fx, fy, fz, m[0], m[1], m[2], m[3]);
+    // the encoding products in one instruction for both nodes; E3M12's results are subnormal floats,
+    // with which the packed product is slower than two scalar ones (778 against 671 us on 256^3)
+#pragma unroll
+    for (int d = 0; d < 27; ++d) {
+        if constexpr (Codec<S>::kPackedScale)
+            f[d] = f[d] * f2(Codec<S>::enc_scale(d));
+        fa[d] = f[d].v.x;
+        fb[d] = f[d].v.y;
+        if constexpr (Codec<S>::kPairs && !Codec<S>::kPackedScale) {
+            fa[d] *= Codec<S>::enc_scale(d);
+            fb[d] *= Codec<S>::enc_scale(d);
+        }
+    }
+    if (a)
+        scatter_scaled<S, EVEN>(planes, na, fa);
+    if (b)
+        scatter_scaled<S, EVEN>(planes, nb, fb);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        mac[0][j] = m[j].v.x;
+        mac[1][j] = m[j].v.y;
     }
 }
 
@@ -267,9 +386,8 @@ __global__ void __launch_bounds__(128) k17_list_kernel(ListCollideArgs<typename 
     } else {
         list_nodes(k, a.nbx, a.nby, a.nbz, a.n, nodes);
     }
-    S *base = static_cast<S *>(a.dist);
     C f[27];
-    gather_pre<S, EVEN>(base, a.n, nodes, f);
+    gather_planes<S, EVEN>(planes_of<S, EXACT>(a.planes, a.n), nodes, f);
     C drho, vx, vy, vz;
     collide<C, EXACT>(f, a.rates, fx, fy, fz, drho, vx, vy, vz);
     if (WRITE_MACRO) {
@@ -278,7 +396,7 @@ __global__ void __launch_bounds__(128) k17_list_kernel(ListCollideArgs<typename 
         a.vz[k] = vz;
         a.rho[k] = drho;
     }
-    scatter_post<S, EVEN>(base, a.n, nodes, f);
+    scatter_planes<S, EVEN>(planes_of<S, EXACT>(a.planes, a.n), nodes, f);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -331,7 +449,6 @@ __global__ void __launch_bounds__(128) k17_list_staged_kernel(ListCollideArgs<ty
         if (t < ntiles)
             list_issue_tile(a.slots, a.slots_stride, t, tiles[warp][s], &bar[s], lane);
     }
-    S *base = static_cast<S *>(a.dist);
     uint32_t parity = 0;
     bool failed = false;
     int it = 0;
@@ -356,10 +473,10 @@ __global__ void __launch_bounds__(128) k17_list_staged_kernel(ListCollideArgs<ty
             list_issue_tile(a.slots, a.slots_stride, tn, tiles[warp][s], &bar[s], lane);
         if ((uint64_t)t * T::N + lane < a.n_idx) {
             C f[27];
-            gather_pre<S, EVEN>(base, a.n, nodes, f);
+            gather_planes<S, EVEN>(a.planes, nodes, f);
             C drho, vx, vy, vz;
             collide<C, EXACT>(f, a.rates, a.fx, a.fy, a.fz, drho, vx, vy, vz);
-            scatter_post<S, EVEN>(base, a.n, nodes, f);
+            scatter_planes<S, EVEN>(a.planes, nodes, f);
         }
     }
     if (failed) {
@@ -423,7 +540,7 @@ __device__ __forceinline__ void store_energy_partial(double *partials, double m,
     }
 }
 
-template <class S, bool EXACT, bool EVEN, bool MASK, bool ENERGY, bool NARROW>
+template <class S, bool EXACT, bool EVEN, bool MASK, bool ENERGY>
 __global__ void __launch_bounds__(128, box_min_blocks<S>()) k17_box_kernel(BoxCollideArgs<typename Codec<S>::compute> a)
 {
     chain_begin();
@@ -438,11 +555,10 @@ __global__ void __launch_bounds__(128, box_min_blocks<S>()) k17_box_kernel(BoxCo
     if (active) {
         uint32_t nodes[8];
         box_slots(a, k, nodes);
-        S *base = static_cast<S *>(a.dist);
         C f[27];
-        gather_pre<S, EVEN, NARROW>(base, a.pitch, nodes, f);
+        gather_planes<S, EVEN>(planes_of<S, EXACT>(a.planes, a.pitch), nodes, f);
         collide<C, EXACT>(f, a.rates, a.fx, a.fy, a.fz, drho, vx, vy, vz);
-        scatter_post<S, EVEN, NARROW>(base, a.pitch, nodes, f);
+        scatter_planes<S, EVEN>(planes_of<S, EXACT>(a.planes, a.pitch), nodes, f);
     }
     if (ENERGY)
         store_energy_partial(a.energy_partials, active ? 1.0 + (double)drho : 0.0,
@@ -638,22 +754,7 @@ __global__ void __launch_bounds__(128, 4) k17_box_pair_kernel(BoxCollideArgs<flo
     }
     float mac[2][4] = { { 0.f, 0.f, 0.f, 0.f }, { 0.f, 0.f, 0.f, 0.f } };
     if (act[0] || act[1]) {
-        S *base = static_cast<S *>(a.dist);
-        float fa[27], fb[27];
-        // an inactive partner collides a rest state (drho = 0, u = 0): finite, never stored
-        if (act[0]) gather_pre<S, EVEN, true>(base, a.pitch, nodes[0], fa);
-        else
-#pragma unroll
-            for (int d = 0; d < 27; ++d) fa[d] = 0.f;
-        if (act[1]) gather_pre<S, EVEN, true>(base, a.pitch, nodes[1], fb);
-        else
-#pragma unroll
-            for (int d = 0; d < 27; ++d) fb[d] = 0.f;
-        collide_pair(fa, fb, a.rates, a.fx, a.fy, a.fz, mac[0], mac[1]);
-        if (act[0])
-            scatter_post<S, EVEN, true>(base, a.pitch, nodes[0], fa);
-        if (act[1])
-            scatter_post<S, EVEN, true>(base, a.pitch, nodes[1], fb);
+        collide_two<S, EVEN>(a.planes, nodes[0], nodes[1], act[0], act[1], a.rates, a.fx, a.fy, a.fz, mac);
     }
     if (ENERGY) {
         double m = 0.0, e = 0.0;
@@ -1923,9 +2024,8 @@ struct PoolNodeCtx {
     C fx, fy, fz;
 };
 template <class C>
-__device__ __forceinline__ PoolNodeCtx<C> load_pool_ctx(const PoolDomain<C> *p)
+__device__ __forceinline__ void load_pool_ctx(const PoolDomain<C> *p, PoolNodeCtx<C> &c)
 {
-    PoolNodeCtx<C> c;
     c.pitch = __ldg(&p->pitch);
     c.nx = __ldg(&p->nx);
     c.ny = __ldg(&p->ny);
@@ -1944,7 +2044,6 @@ __device__ __forceinline__ PoolNodeCtx<C> load_pool_ctx(const PoolDomain<C> *p)
     c.fx = __ldg(&p->fx);
     c.fy = __ldg(&p->fy);
     c.fz = __ldg(&p->fz);
-    return c;
 }
 
 // the slot nodes of node k of a pool domain
@@ -1971,13 +2070,13 @@ __device__ __forceinline__ void pool_slots(const PoolNodeCtx<C> &dm, uint32_t k,
 }
 
 // nodes a thread collides together: two in packed FP32x2 arithmetic (the FP32-arithmetic forms), else
-// one. NARROW: every domain's planes stay below 4 GB (slot_at)
+// one. NARROW: every domain's planes stay below 4 GB (PlaneNarrow)
 template <class S, bool EXACT, bool NARROW>
 constexpr int pool_width() { return sizeof(typename Codec<S>::compute) == 4 && !EXACT && NARROW ? 2 : 1; }
 
 // the slots, the K17 collision and the ET scatter of a thread's nodes of a pool domain
-template <class S, bool EXACT, bool EVEN, bool NARROW, int W>
-__device__ __forceinline__ void pool_collide_nodes(S *base, const PoolNodeCtx<typename Codec<S>::compute> &dm,
+template <class S, bool EXACT, bool EVEN, int W, class P>
+__device__ __forceinline__ void pool_collide_nodes(const P &planes, const PoolNodeCtx<typename Codec<S>::compute> &dm,
                                                    const uint32_t (&k)[W], const bool (&act)[W])
 {
     using C = typename Codec<S>::compute;
@@ -1987,31 +2086,18 @@ __device__ __forceinline__ void pool_collide_nodes(S *base, const PoolNodeCtx<ty
         uint32_t nodes[8];
         pool_slots(dm, k[0], nodes);
         C f[27];
-        gather_pre<S, EVEN, NARROW>(base, dm.pitch, nodes, f);
+        gather_planes<S, EVEN>(planes, nodes, f);
         C drho, vx, vy, vz;
         collide<C, EXACT>(f, dm.rates, dm.fx, dm.fy, dm.fz, drho, vx, vy, vz);
-        scatter_post<S, EVEN, NARROW>(base, dm.pitch, nodes, f);
+        scatter_planes<S, EVEN>(planes, nodes, f);
     } else {
         if (!act[0] && !act[1])
             return;
         uint32_t na[8], nb[8];
         pool_slots(dm, k[0], na);
         pool_slots(dm, k[1], nb);
-        // an inactive partner collides a rest state: finite, never stored
-        float fa[27], fb[27], ma[4], mb[4];
-        if (act[0]) gather_pre<S, EVEN, NARROW>(base, dm.pitch, na, fa);
-        else
-#pragma unroll
-            for (int d = 0; d < 27; ++d) fa[d] = 0.f;
-        if (act[1]) gather_pre<S, EVEN, NARROW>(base, dm.pitch, nb, fb);
-        else
-#pragma unroll
-            for (int d = 0; d < 27; ++d) fb[d] = 0.f;
-        collide_pair(fa, fb, dm.rates, dm.fx, dm.fy, dm.fz, ma, mb);
-        if (act[0])
-            scatter_post<S, EVEN, NARROW>(base, dm.pitch, na, fa);
-        if (act[1])
-            scatter_post<S, EVEN, NARROW>(base, dm.pitch, nb, fb);
+        float mac[2][4];
+        collide_two<S, EVEN>(planes, na, nb, act[0], act[1], dm.rates, dm.fx, dm.fy, dm.fz, mac);
     }
 }
 
@@ -2045,11 +2131,11 @@ __global__ void __launch_bounds__(256, pool_min_blocks<S>()) k17_pool_kernel(Poo
         const PoolDomain<C> *dp = a.domains + it.x;
         __syncthreads();                 // every thread is done with the previous item's record
         if (threadIdx.x == 0)
-            ctx = load_pool_ctx(dp);
+            load_pool_ctx(dp, ctx);
         __syncthreads();
         const PoolNodeCtx<C> &dm = ctx;
         const uint32_t nodes_total = (uint32_t)dm.nx * (uint32_t)dm.ny * (uint32_t)dm.nz;
-        S *base = static_cast<S *>(a.arena) + __ldg(&dp->dist_offset);
+        const std::conditional_t<NARROW, PlaneNarrow, PlaneStride> planes{ static_cast<S *>(a.arena) + __ldg(&dp->dist_offset), dm.pitch };
         const uint32_t end = min(it.y + span, nodes_total);
         const uint8_t *mask =
             (dm.flags & kPoolMask) ? static_cast<const uint8_t *>(a.arena) + __ldg(&dp->mask_offset) : nullptr;
@@ -2099,7 +2185,7 @@ __global__ void __launch_bounds__(256, pool_min_blocks<S>()) k17_pool_kernel(Poo
                     q[lane] = rest;
                 pending = left;
             }
-            pool_collide_nodes<S, EXACT, EVEN, NARROW, W>(base, dm, k, act);
+            pool_collide_nodes<S, EXACT, EVEN, W>(planes, dm, k, act);
         }
         __syncwarp();
     }

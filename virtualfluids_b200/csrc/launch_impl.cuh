@@ -38,6 +38,14 @@ inline void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, cud
     c.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
     cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
+template <class S>
+PlaneTable plane_table(void *dist, uint64_t n)
+{
+    PlaneTable t;
+    for (int i = 0; i < 27; ++i)
+        t.p[i] = static_cast<S *>(dist) + (uint64_t)i * n;
+    return t;
+}
 inline unsigned grid1d(uint64_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
 
 template <class C>
@@ -65,7 +73,7 @@ cudaError_t Launchers<S>::k17_list(const vfb_level *L, const uint32_t *idx, uint
     if (n == 0)
         return cudaSuccess;
     ListCollideArgs<C> a;
-    a.dist = L->distributions;
+    a.planes = plane_table<S>(L->distributions, L->number_of_nodes);
     a.n = L->number_of_nodes;
     a.nbx = L->neighbor_x;
     a.nby = L->neighbor_y;
@@ -120,7 +128,7 @@ cudaError_t Launchers<S>::k17_list_staged(const vfb_level *L, const uint32_t *sl
     if (n == 0)
         return cudaSuccess;
     ListCollideArgs<C> a{};
-    a.dist = L->distributions;
+    a.planes = plane_table<S>(L->distributions, L->number_of_nodes);
     a.n = L->number_of_nodes;
     a.n_idx = n;
     a.slots = slots;
@@ -559,12 +567,14 @@ cudaError_t Launchers<S>::energy_list(const vfb_level *L, const uint32_t *idx, u
 }
 
 namespace {
-template <class C>
-BoxCollideArgs<C> box_args(const BoxState &b)
+template <class S>
+BoxCollideArgs<typename Codec<S>::compute> box_args(const BoxState &b)
 {
+    using C = typename Codec<S>::compute;
     BoxCollideArgs<C> a;
     a.dist = b.dist;
     a.pitch = b.pitch;
+    a.planes = plane_table<S>(b.dist, b.pitch);
     a.nx = b.nx;
     a.ny = b.ny;
     a.nz = b.nz;
@@ -722,35 +732,24 @@ cudaError_t launch_box_pipe(const BoxCollideArgs<typename Codec<S>::compute> &a,
         *n_partials = (uint64_t)grid * (uint64_t)(B / 32);
     return cudaGetLastError();
 }
-// one node per thread; FP64 takes 64-bit slot addresses (its registers allow them)
+// one node per thread
 template <class S>
-void launch_box_direct(const BoxCollideArgs<typename Codec<S>::compute> &a, bool even, bool narrow, unsigned G, unsigned B,
-                       cudaStream_t s)
+void launch_box_direct(const BoxCollideArgs<typename Codec<S>::compute> &a, bool even, unsigned G, unsigned B, cudaStream_t s)
 {
     const bool mask = a.mask != nullptr, energy = a.energy_partials != nullptr;
-    auto launch = [&](auto narrow_planes_c) {
-        constexpr bool W = decltype(narrow_planes_c)::value;
-#define VFB_K17B(E, M, N) launch_next(k17_box_kernel<S, VFB_EXACT, E, M, N, W>, G, B, s, a)
-        if (even) {
-            if (mask && energy) VFB_K17B(true, true, true);
-            else if (mask) VFB_K17B(true, true, false);
-            else if (energy) VFB_K17B(true, false, true);
-            else VFB_K17B(true, false, false);
-        } else {
-            if (mask && energy) VFB_K17B(false, true, true);
-            else if (mask) VFB_K17B(false, true, false);
-            else if (energy) VFB_K17B(false, false, true);
-            else VFB_K17B(false, false, false);
-        }
-#undef VFB_K17B
-    };
-    if constexpr (sizeof(S) <= 4) {
-        if (narrow) {
-            launch(std::true_type{});
-            return;
-        }
+#define VFB_K17B(E, M, N) launch_next(k17_box_kernel<S, VFB_EXACT, E, M, N>, G, B, s, a)
+    if (even) {
+        if (mask && energy) VFB_K17B(true, true, true);
+        else if (mask) VFB_K17B(true, true, false);
+        else if (energy) VFB_K17B(true, false, true);
+        else VFB_K17B(true, false, false);
+    } else {
+        if (mask && energy) VFB_K17B(false, true, true);
+        else if (mask) VFB_K17B(false, true, false);
+        else if (energy) VFB_K17B(false, false, true);
+        else VFB_K17B(false, false, false);
     }
-    launch(std::false_type{});
+#undef VFB_K17B
 }
 } // namespace
 
@@ -758,7 +757,7 @@ template <class S>
 cudaError_t Launchers<S>::box_collide(const BoxState &b, bool even, double *partials, uint64_t *n_partials, cudaStream_t s)
 {
     using C = typename Codec<S>::compute;
-    BoxCollideArgs<C> a = box_args<C>(b);
+    BoxCollideArgs<C> a = box_args<S>(b);
     a.energy_partials = partials;
     const bool mask = b.mask != nullptr, energy = partials != nullptr;
     if constexpr (sizeof(S) >= 4) {
@@ -797,7 +796,7 @@ cudaError_t Launchers<S>::box_collide(const BoxState &b, bool even, double *part
         // two nodes per thread where they fill the device: 148 SMs x 4 blocks x 256 nodes. Below
         // that one node per thread spreads the box over more warps (32^3 in FP32: 4.1 against 6.2 us
         // per step; 64^3: equal)
-        if (narrow_planes(b.pitch, sizeof(S)) && (b.variant == 4 || (b.variant == 0 && a.count >= 148u * 4u * 256u))) {
+        if (b.variant == 4 || (b.variant == 0 && a.count >= 148u * 4u * 256u)) {
             const unsigned B = box_threads(a.count / 2), G = grid1d(((uint64_t)a.count + 1) / 2, B);
             if (n_partials)
                 *n_partials = (uint64_t)G * (B / 32);
@@ -836,7 +835,7 @@ cudaError_t Launchers<S>::box_collide(const BoxState &b, bool even, double *part
     const unsigned B = box_threads(a.count), G = grid1d(a.count, B);
     if (n_partials)
         *n_partials = (uint64_t)G * (B / 32);
-    launch_box_direct<S>(a, even, narrow_planes(b.pitch, sizeof(S)), G, B, s);
+    launch_box_direct<S>(a, even, G, B, s);
     return cudaGetLastError();
 }
 
@@ -866,11 +865,11 @@ cudaError_t Launchers<S>::box_collide_planes(const BoxState &b, bool even, int z
     using C = typename Codec<S>::compute;
     if (z1 <= z0)
         return cudaSuccess;
-    BoxCollideArgs<C> a = box_args<C>(b);
+    BoxCollideArgs<C> a = box_args<S>(b);
     a.first = (uint32_t)((uint64_t)b.nx * b.ny * z0);
     a.count = (uint32_t)((uint64_t)b.nx * b.ny * (z1 - z0));
     const unsigned B = box_threads(a.count), G = grid1d(a.count, B);
-    launch_box_direct<S>(a, even, narrow_planes(b.pitch, sizeof(S)), G, B, s);
+    launch_box_direct<S>(a, even, G, B, s);
     return cudaGetLastError();
 }
 
@@ -878,7 +877,7 @@ template <class S>
 cudaError_t Launchers<S>::box_collide_border(const BoxState &b, bool even, int z, void *up, void *down, cudaStream_t s)
 {
     using C = typename Codec<S>::compute;
-    BoxCollideArgs<C> a = box_args<C>(b);
+    BoxCollideArgs<C> a = box_args<S>(b);
     dim3 G = box_grid(b);
     G.z = 1;
     const dim3 B(box_block_x(b.nx));
@@ -899,7 +898,7 @@ cudaError_t Launchers<S>::box_init(const BoxState &b, bool even, const void *rho
                                    const void *uz, cudaStream_t s)
 {
     using C = typename Codec<S>::compute;
-    BoxCollideArgs<C> a = box_args<C>(b);
+    BoxCollideArgs<C> a = box_args<S>(b);
     const unsigned B = box_threads(a.count), G = grid1d(a.count, B);
     if (even) init_box_kernel<S, true><<<G, B, 0, s>>>(a, rho, ux, uy, uz);
     else init_box_kernel<S, false><<<G, B, 0, s>>>(a, rho, ux, uy, uz);
@@ -910,7 +909,7 @@ template <class S>
 cudaError_t Launchers<S>::box_macros(const BoxState &b, bool even, void *rho, void *ux, void *uy, void *uz, cudaStream_t s)
 {
     using C = typename Codec<S>::compute;
-    BoxCollideArgs<C> a = box_args<C>(b);
+    BoxCollideArgs<C> a = box_args<S>(b);
     a.rho = static_cast<C *>(rho);
     a.vx = static_cast<C *>(ux);
     a.vy = static_cast<C *>(uy);

@@ -1,6 +1,6 @@
 // Packed FP32x2 arithmetic for sm_100a: two independent nodes' values in one 64-bit register pair,
-// every add, multiply and fused multiply-add issued as one instruction for both (the sm_100
-// __fadd2_rn / __fmul2_rn / __ffma2_rn operations, each lane rounded as the scalar operation).
+// every add, multiply and fused multiply-add issued as one instruction for both (sm_100's f32x2
+// operations, each lane rounded as the scalar operation).
 // The K17 collision is generic over its arithmetic type, so instantiated with f2 it collides two
 // nodes per thread at half the instruction count of the arithmetic, each node with the bits of the
 // scalar form.
@@ -42,25 +42,6 @@ __host__ __device__ __forceinline__ void limiter_inverses(const f2 (&m)[7], cons
 #pragma unroll
     for (int i = 0; i < 7; ++i)
         iv[i] = f2(k17detail::fast_rcp(rn_add(fabsf(m[i].v.x), q[i])), k17detail::fast_rcp(rn_add(fabsf(m[i].v.y), q[i])));
-}
-
-// two nodes' K17 collisions (the fast arithmetic) with packed operations; fa, fb in place
-__device__ __forceinline__ void collide_pair(float (&fa)[27], float (&fb)[27], const K17Rates<float> &r, float fx,
-                                             float fy, float fz, float (&ma)[4], float (&mb)[4])
-{
-    f2 f[27];
-#pragma unroll
-    for (int d = 0; d < 27; ++d)
-        f[d] = f2(fa[d], fb[d]);
-    f2 drho, vx, vy, vz;
-    k17_collide_fast<f2, float>(f, r, fx, fy, fz, drho, vx, vy, vz);
-#pragma unroll
-    for (int d = 0; d < 27; ++d) {
-        fa[d] = f[d].v.x;
-        fb[d] = f[d].v.y;
-    }
-    ma[0] = drho.v.x; ma[1] = vx.v.x; ma[2] = vy.v.x; ma[3] = vz.v.x;
-    mb[0] = drho.v.y; mb[1] = vx.v.y; mb[2] = vy.v.y; mb[3] = vz.v.y;
 }
 
 } // namespace vfb

@@ -32,24 +32,6 @@ enum StorageKind : int { kStoreF64 = 0, kStoreF32 = 1, kStoreF16 = 2, kStoreBF16
 template <class S>
 struct Codec;
 
-// Node k's slot in a direction plane. NARROW (narrow_planes, addr.h): planes below 4 GB; the byte offset is a 32-bit product
-// added to the plane's pointer, which is the same for every thread. It needs one register per slot
-// class where 64-bit sums need two (the two-node FP32 kernel spilled 28-68 bytes with them at its
-// 128 registers, and took 671 instead of 589 us on 320 x 256 x 192).
-template <bool NARROW, class S>
-__device__ __forceinline__ S *slot_at(S *plane, uint32_t k)
-{
-    if constexpr (NARROW)
-        return reinterpret_cast<S *>(reinterpret_cast<char *>(plane) + k * (uint32_t)sizeof(S));
-    else
-        return plane + k;
-}
-template <bool NARROW, class S>
-__device__ __forceinline__ const S *slot_at(const S *plane, uint32_t k)
-{
-    return slot_at<NARROW>(const_cast<S *>(plane), k);
-}
-
 // float(1 / w_d) for a run-time d: the constants the 16-bit stores scale by
 __device__ __forceinline__ float inv_weight_rt(int d)
 {
@@ -73,6 +55,7 @@ struct Codec<float> {
     using compute = float;
     static constexpr bool kPairs = false;
     __device__ __forceinline__ static float load(const float *p, int) { return *p; }
+    static constexpr bool kPackedScale = false;
     __device__ __forceinline__ static void store(float *p, float v, int) { *p = v; }
     __device__ __forceinline__ static void store_at(float *base, uint64_t off, float v, int) { base[off] = v; }
     __device__ __forceinline__ static void store_at_rt(float *base, uint64_t off, float v, int) { base[off] = v; }
@@ -88,15 +71,15 @@ struct Codec<float> {
 __device__ __forceinline__ uint32_t sr_bits(float v, uint32_t off)
 {
     // two odd multipliers carry the value's (noisy) low mantissa bits and the slot offset (its low 32
-    // bits) into every bit position; sums of products, because the 16-bit forms are bound by the
-    // instructions they issue: with off = plane + node, each product with the rest of the sum is
-    // one multiply-add
+    // bits) into every bit position
     return __float_as_uint(v) * 0x9E3779B1u + off * 0x85EBCA77u;
 }
-// the bits of two values rounded together: the first one's, moved by the second value
-__device__ __forceinline__ uint32_t sr_bits(float v0, float v1, uint32_t off0)
+// the collision's bits for two values rounded together: node k and plane p of the first one's slot, and
+// both values. A sum of products: the 16-bit forms are bound by the instructions they issue, and
+// each product is one multiply-add with the rest of the sum.
+__device__ __forceinline__ uint32_t sr_bits(float v0, float v1, uint32_t k, int p)
 {
-    return __float_as_uint(v1) * 0xC2B2AE35u + sr_bits(v0, off0);
+    return __float_as_uint(v1) * 0xC2B2AE35u + (__float_as_uint(v0) * 0x9E3779B1u + (k * 0x85EBCA77u + (uint32_t)p * 0x632BE5ABu));
 }
 
 __device__ __forceinline__ __half half_sr(float v, uint32_t rbits)
@@ -132,22 +115,25 @@ template <>
 struct Codec<__half> {
     using compute = float;
     static constexpr bool kPairs = true;
-    // two slots, node k of the plane at p each; off0: slot p0's plane in its array (low 32 bits)
-    template <bool NARROW>
-    __device__ __forceinline__ static void store_pair(__half *p0, uint32_t k0, uint32_t off0, float v0, int d0, __half *p1,
-                                                      uint32_t k1, float v1, int d1)
+    static constexpr bool kPackedScale = true;
+    __device__ __forceinline__ static constexpr float enc_scale(int d) { return float(1.0 / weight(d)); }
+    // two scaled values into two slots; node k0 of plane plane0: the first one's place
+    __device__ __forceinline__ static void store_pair(__half *p0, uint32_t k0, int plane0, float s0, __half *p1, float s1)
     {
-        const float s0 = v0 * float(1.0 / weight(d0)), s1 = v1 * float(1.0 / weight(d1));
-        const uint32_t h = half2_sr(s0, s1, sr_bits(s0, s1, off0 + k0));
-        *slot_at<NARROW>(p0, k0) = __ushort_as_half((unsigned short)(h >> 16));
-        *slot_at<NARROW>(p1, k1) = __ushort_as_half((unsigned short)(h & 0xffffu));
+        const uint32_t h = half2_sr(s0, s1, sr_bits(s0, s1, k0, plane0));
+        *p0 = __ushort_as_half((unsigned short)(h >> 16));
+        *p1 = __ushort_as_half((unsigned short)(h & 0xffffu));
     }
     // the decoding product is rounded on its own (never fused into a later addition), so a decoded
     // value is the same float wherever it is used or saved
     __device__ __forceinline__ static float load(const __half *p, int d) { return __fmul_rn(__half2float(*p), float(weight(d))); }
+    __device__ __forceinline__ static void store_scaled(__half *p, uint32_t k, int plane, float s)
+    {
+        *p = half_sr(s, sr_bits(s, 0.0f, k, plane));
+    }
     __device__ __forceinline__ static void store_at(__half *base, uint64_t off, float v, int d)
     {
-        const float s = v * float(1.0 / weight(d));
+        const float s = v * enc_scale(d);
         base[off] = half_sr(s, sr_bits(s, (uint32_t)off));
     }
     // store_at for a direction known only at run time (the same scale factors)
@@ -162,23 +148,26 @@ template <>
 struct Codec<__nv_bfloat16> {
     using compute = float;
     static constexpr bool kPairs = true;
-    // two slots, node k of the plane at p each; off0: slot p0's plane in its array (low 32 bits)
-    template <bool NARROW>
-    __device__ __forceinline__ static void store_pair(__nv_bfloat16 *p0, uint32_t k0, uint32_t off0, float v0, int d0, __nv_bfloat16 *p1,
-                                                      uint32_t k1, float v1, int d1)
+    static constexpr bool kPackedScale = true;
+    __device__ __forceinline__ static constexpr float enc_scale(int d) { return float(1.0 / weight(d)); }
+    // two scaled values into two slots; node k0 of plane plane0: the first one's place
+    __device__ __forceinline__ static void store_pair(__nv_bfloat16 *p0, uint32_t k0, int plane0, float s0, __nv_bfloat16 *p1, float s1)
     {
-        const float s0 = v0 * float(1.0 / weight(d0)), s1 = v1 * float(1.0 / weight(d1));
-        const uint32_t h = bf162_sr(s0, s1, sr_bits(s0, s1, off0 + k0));
-        *slot_at<NARROW>(p0, k0) = __ushort_as_bfloat16((unsigned short)(h >> 16));
-        *slot_at<NARROW>(p1, k1) = __ushort_as_bfloat16((unsigned short)(h & 0xffffu));
+        const uint32_t h = bf162_sr(s0, s1, sr_bits(s0, s1, k0, plane0));
+        *p0 = __ushort_as_bfloat16((unsigned short)(h >> 16));
+        *p1 = __ushort_as_bfloat16((unsigned short)(h & 0xffffu));
     }
     __device__ __forceinline__ static float load(const __nv_bfloat16 *p, int d)
     {
         return __fmul_rn(__bfloat162float(*p), float(weight(d)));   // rounded on its own, as for FP16
     }
+    __device__ __forceinline__ static void store_scaled(__nv_bfloat16 *p, uint32_t k, int plane, float s)
+    {
+        *p = bf16_sr(s, sr_bits(s, 0.0f, k, plane));
+    }
     __device__ __forceinline__ static void store_at(__nv_bfloat16 *base, uint64_t off, float v, int d)
     {
-        const float s = v * float(1.0 / weight(d));
+        const float s = v * enc_scale(d);
         base[off] = bf16_sr(s, sr_bits(s, (uint32_t)off));
     }
     __device__ __forceinline__ static void store_at_rt(__nv_bfloat16 *base, uint64_t off, float v, int d)
@@ -254,24 +243,27 @@ template <>
 struct Codec<e3m12_t> {
     using compute = float;
     static constexpr bool kPairs = true;
+    static constexpr bool kPackedScale = false;
     // (1/w) 2^-120 and w 2^120 for direction d: power-of-two scalings of the other 16-bit forms'
     // float constants, folded into their one multiplication
     __device__ __forceinline__ static float enc_scale(int d) { return float(1.0 / weight(d)) * 0x1p-120f; }
     __device__ __forceinline__ static float dec_scale(int d) { return float(weight(d)) * 0x1p120f; }
-    template <bool NARROW>
-    __device__ __forceinline__ static void store_pair(e3m12_t *p0, uint32_t k0, uint32_t off0, float v0, int d0,
-                                                      e3m12_t *p1, uint32_t k1, float v1, int d1)
+    __device__ __forceinline__ static void store_pair(e3m12_t *p0, uint32_t k0, int plane0, float t0,
+                                                      e3m12_t *p1, float t1)
     {
-        const float t0 = v0 * enc_scale(d0), t1 = v1 * enc_scale(d1);
         // 11 random bits each from the upper bits of the hash (they mix all of the value's bits)
-        const uint32_t r = sr_bits(t0, t1, off0 + k0);
-        slot_at<NARROW>(p0, k0)->bits = e3m12::encode_scaled(t0, r >> 21);
-        slot_at<NARROW>(p1, k1)->bits = e3m12::encode_scaled(t1, (r >> 10) & 0x7ffu);
+        const uint32_t r = sr_bits(t0, t1, k0, plane0);
+        p0->bits = e3m12::encode_scaled(t0, r >> 21);
+        p1->bits = e3m12::encode_scaled(t1, (r >> 10) & 0x7ffu);
     }
     // rounded on its own, as for the other 16-bit forms
     __device__ __forceinline__ static float load(const e3m12_t *p, int d)
     {
         return __fmul_rn(e3m12::decode_scaled(p->bits), dec_scale(d));
+    }
+    __device__ __forceinline__ static void store_scaled(e3m12_t *p, uint32_t k, int plane, float t)
+    {
+        p->bits = e3m12::encode_scaled(t, sr_bits(t, 0.0f, k, plane) >> 21);
     }
     __device__ __forceinline__ static void store_at(e3m12_t *base, uint64_t off, float v, int d)
     {

@@ -1836,10 +1836,12 @@ __global__ void __launch_bounds__(128) scale_cf_kernel(ScaleArgs a)
     const uint64_t cell = t >> 3;
     const int corner = (int)(t & 7u);
     const bool valid = cell < a.n_cells;
-    uint32_t k = 0;
+    uint32_t k = 0, nodes[8];   // the target's slots are looked up with the source's: two chains of dependent loads at once
     C xo = C(0), yo = C(0), zo = C(0);
     if (valid) {
         k = cell_corner(__ldg(a.coarse_cells + cell), corner, a.nbx_c, a.nby_c, a.nbz_c, a.n_coarse);
+        list_nodes(cell_corner(__ldg(a.fine_cells + cell), corner, a.nbx_f, a.nby_f, a.nbz_f, a.n_fine), a.nbx_f, a.nby_f,
+                   a.nbz_f, a.n_fine, nodes);
         xo = static_cast<const C *>(a.ox)[cell];
         yo = static_cast<const C *>(a.oy)[cell];
         zo = static_cast<const C *>(a.oz)[cell];
@@ -1853,9 +1855,6 @@ __global__ void __launch_bounds__(128) scale_cf_kernel(ScaleArgs a)
     C f[27];
     interp_point<C, false>(coef, (C)a.omega_fine, C(0.5), (corner & 1) ? q : -q, (corner & 2) ? q : -q,
                            (corner & 4) ? q : -q, f);
-    uint32_t nodes[8];
-    list_nodes(cell_corner(__ldg(a.fine_cells + cell), corner, a.nbx_f, a.nby_f, a.nbz_f, a.n_fine), a.nbx_f, a.nby_f,
-               a.nbz_f, a.n_fine, nodes);
     S *fine = static_cast<S *>(a.dist_fine);
 #pragma unroll
     for (int d = 0; d < 27; ++d)
@@ -1875,10 +1874,11 @@ __global__ void __launch_bounds__(128) scale_fc_kernel(ScaleArgs a)
     const uint64_t cell = t >> 3;
     const int corner = (int)(t & 7u);
     const bool valid = cell < a.n_cells;
-    uint32_t k = 0;
+    uint32_t k = 0, nodes[8];   // the target's slots are looked up with the source's: two chains of dependent loads at once
     C xo = C(0), yo = C(0), zo = C(0);
     if (valid) {
         k = cell_corner(__ldg(a.fine_cells + cell), corner, a.nbx_f, a.nby_f, a.nbz_f, a.n_fine);
+        list_nodes(__ldg(a.coarse_cells + cell), a.nbx_c, a.nby_c, a.nbz_c, a.n_coarse, nodes);
         xo = static_cast<const C *>(a.ox)[cell];
         yo = static_cast<const C *>(a.oy)[cell];
         zo = static_cast<const C *>(a.oz)[cell];
@@ -1890,8 +1890,6 @@ __global__ void __launch_bounds__(128) scale_fc_kernel(ScaleArgs a)
         return;
     C f[27];
     interp_point<C, true>(coef, (C)a.omega_coarse, C(2), C(0), C(0), C(0), f);
-    uint32_t nodes[8];
-    list_nodes(__ldg(a.coarse_cells + cell), a.nbx_c, a.nby_c, a.nbz_c, a.n_coarse, nodes);
     S *coarse = static_cast<S *>(a.dist_coarse);
 #pragma unroll
     for (int d = 0; d < 27; ++d)

@@ -399,6 +399,29 @@ __global__ void __launch_bounds__(128) k17_list_kernel(ListCollideArgs<typename 
     scatter_planes<S, EVEN>(planes_of<S, EXACT>(a.planes, a.n), nodes, f);
 }
 
+// The default collision of the FP32-arithmetic forms over a slot table with two list entries per thread,
+// 32 apart (collide_two): the bits of k17_list_kernel.
+template <class S, bool EVEN>
+__global__ void __launch_bounds__(128, 4) k17_list_pair_kernel(ListCollideArgs<float> a)
+{
+    chain_begin();
+    const uint32_t i0 = 2u * (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) + (threadIdx.x & 31u);
+    const bool act[2] = { i0 < a.n_idx, i0 + 32u < a.n_idx };
+    uint32_t nodes[2][8];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const uint32_t i = act[p] ? i0 + 32u * p : 0u;
+        nodes[p][0] = VFB_NODE(__ldg(a.idx + i), a.n);
+#pragma unroll
+        for (int j = 1; j < 8; ++j)
+            nodes[p][j] = VFB_NODE(__ldg(a.slots + (size_t)j * a.slots_stride + i), a.n);
+    }
+    if (!act[0])
+        return;
+    float mac[2][4];
+    collide_two<S, EVEN>(a.planes, nodes[0], nodes[1], act[0], act[1], a.rates, a.fx, a.fy, a.fz, mac);
+}
+
 // ---------------------------------------------------------------------------------------------
 // The same collision over the reference layout with the slot table staged in shared memory: every
 // warp walks tiles of 32 list entries and keeps the eight node indices of its next two tiles in
@@ -2402,8 +2425,8 @@ __global__ void __launch_bounds__(128) pool_pressure_kernel(PoolBCArgs<typename 
         const C *rho = reinterpret_cast<const C *>(arena + dm.pressure_rho_offset);
         const NodeAddr box{ dm.nx, dm.ny, dm.nz, dm.flags & 7 };
         uint32_t nk[8], nn[8];
-        box_nodes((uint32_t)k[i], box, nk);
-        box_nodes((uint32_t)kn[i], box, nn);
+        box_nodes((uint32_t)k[i], box, dm.div_nx, dm.div_ny, nk);
+        box_nodes((uint32_t)kn[i], box, dm.div_nx, dm.div_ny, nn);
         bc_pressure_neq_node<S, EVEN, false>(static_cast<S *>(a.arena) + dm.dist_offset, dm.pitch, nk, nn, rho[i],
                                              dir[i]);
     }

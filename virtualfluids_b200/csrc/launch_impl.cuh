@@ -102,6 +102,15 @@ cudaError_t Launchers<S>::k17_list(const vfb_level *L, const uint32_t *idx, uint
     const bool bf = tmpl == VFB_COLLISION_APPLY_BODY_FORCE || tmpl == VFB_COLLISION_ALL_FEATURES || tmpl == VFB_COLLISION_SUBDOMAIN_BORDER;
     const unsigned B = 128, G = grid1d(n, B);
     const bool even = L->is_even_timestep != 0;
+    if constexpr (std::is_same<C, float>::value && !VFB_EXACT) {
+        // two entries per thread where they fill the device, as for a box (n < 2^31: 32-bit entry numbers)
+        if (slots && !wm && !bf && n >= 148u * 4u * 256u && n < (1u << 31)) {
+            const unsigned G2 = grid1d(((uint64_t)n + 1) / 2, B);
+            if (even) launch_next(k17_list_pair_kernel<S, true>, G2, B, s, a);
+            else launch_next(k17_list_pair_kernel<S, false>, G2, B, s, a);
+            return cudaGetLastError();
+        }
+    }
 #define VFB_K17L(E, W, F) launch_next(k17_list_kernel<S, VFB_EXACT, E, W, F>, G, B, s, a)
     if (even) {
         if (wm && bf) VFB_K17L(true, true, true);

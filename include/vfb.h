@@ -454,10 +454,10 @@ int vfb_box_fields(vfb_box *box, void *rho, void *ux, void *uy, void *uz, int32_
 /* synchronises the stream and reads the status word the box's kernels set on a failed internal wait
    (0 = fine); returns VFB_ERR_CUDA when it is nonzero */
 int vfb_box_status(vfb_box *box, int32_t *device_status, void *stream);
-/* collision kernel: 0 = choose (direct loads, the fastest measured on B200 for every storage),
-   1 = direct loads, 2 = TMA-staged warp tiles (nx % 32 == 0),
+/* collision kernel: 0 = choose (two nodes per thread for FP32-arithmetic boxes of 151552 nodes and
+   more, else one), 1 = one node per thread, 2 = TMA-staged warp tiles (nx % 32 == 0),
    3 = per-thread asynchronous copies (F64 and F32 storage),
-   4 = two nodes per thread in packed FP32x2 arithmetic (F32, F16, BF16 storage, FMA arithmetic),
+   4 = two nodes per thread in packed FP32x2 arithmetic (FP32 arithmetic; the bits of 1),
    5 = persistent blocks with the next node's loads in flight while the current node is collided */
 int vfb_box_set_kernel_variant(vfb_box *box, int32_t variant);
 /* Boundary conditions on a box, run by vfb_box_step in the order of vfb_simulation_run: velocity,

@@ -98,7 +98,8 @@ class Box:
         return v.value
 
     def set_kernel_variant(self, variant: str):
-        """'auto', 'direct' (plain loads), 'tma' (bulk copies staged in shared memory), 'async'
+        """'auto' (two nodes per thread for FP32-arithmetic boxes that fill the device, else one),
+        'direct' (one node per thread), 'tma' (bulk copies staged in shared memory), 'async'
         (per-thread asynchronous copies of the next node), 'pairs' (two nodes per thread in packed
         FP32x2 arithmetic; FP32-arithmetic forms) or 'pipe' (persistent blocks, the next node's loads
         in flight in registers while the current node is collided)."""

@@ -40,7 +40,8 @@ struct BoxState {
     double omega;
     double fx, fy, fz;            // half acceleration
     double lim[3];
-    int variant;                  // 0: choose, 1: direct loads, 2: TMA-staged (nx % 32 == 0), 3: async copies
+    int variant;                  // 0: choose, 1: one node per thread, 2: TMA-staged (nx % 32 == 0), 3: async copies,
+                                  // 4: two nodes per thread (FP32 arithmetic), 5: persistent pipeline
     int async_blocks_per_sm;      // async kernel: resident blocks per SM (0: 3)
     int async_smem_kb;            // async kernel: shared-memory configuration to pad to (0: carve-out hint only)
     int *status;                  // device status word (DeviceError), nullable

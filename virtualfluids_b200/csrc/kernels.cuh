@@ -229,10 +229,11 @@ __device__ __forceinline__ void node_slots(uint32_t k, const uint32_t *nbx, cons
         box_nodes(k, b, nodes);
 }
 
-// FP64 with FMA arithmetic is bound by memory, and was 6 % slower with the table (256^3 1205 against
-// 1130 us per step); the exact form gains 0.8 % from it
+// Which one-node kernels take the table: the exact FP64 ones (0.8 %). FP64 with FMA arithmetic was 6 %
+// slower with it (256^3 1205 against 1130 us per step), the FP32-arithmetic forms no faster, and a
+// small box lost 4 % to reading 27 pointers per launch (64 steps of 32^3 228 against 220 us).
 template <class S, bool EXACT>
-constexpr bool plane_table_pays() { return sizeof(typename Codec<S>::compute) == 4 || EXACT; }
+constexpr bool plane_table_pays() { return sizeof(S) == 8 && EXACT; }
 template <class S, bool EXACT>
 __device__ __forceinline__ auto planes_of(const PlaneTable &t, uint64_t n)
 {

@@ -1,10 +1,11 @@
 """Quadric limiters far from the default 0.01 on the GPU: infinite, very large (the limiter is off), very
-small. The exact arithmetic computes the oracle's bits with each of them."""
+small. The exact arithmetic computes the oracle's bits with each of them, and the FMA arithmetic one result
+for all that are off."""
 import numpy as np
 import pytest
 
 from virtualfluids_b200 import BoundaryConditionFactory as BCF
-from virtualfluids_b200 import ListGrid, Parameter, Simulation
+from virtualfluids_b200 import Box, ListGrid, Parameter, Simulation
 from virtualfluids_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
@@ -36,3 +37,33 @@ def test_exact_arithmetic_with_any_limiter_matches_the_oracle(oracle, cuda, limi
     orc.init(*f)
     orc.run(6)
     assert np.isfinite(orc.f).all() and np.array_equal(sim.populations(), orc.f)
+
+
+@pytest.mark.parametrize("storage,arith", [("f64", "fast"), ("f32", "fast"), ("f32", "exact"), ("f16", "fast")])
+def test_limiters_that_are_off_give_one_result(cuda, storage, arith):
+    shape, n = (33, 9, 8), 33 * 9 * 8
+    f = _fields(n, 5)
+    out = []
+    for q in (2.0 ** 100, 1e38, np.inf):
+        b = Box(*shape, 1.9, storage=storage, arith=arith, quadric_limiters=(q, q, q))
+        b.init(*f)
+        b.step(5)
+        assert all(np.isfinite(v).all() for v in b.fields().values())
+        out.append(b.read_populations()[0])
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("storage", ["f64", "f32"])
+def test_infinite_limiters_fma_against_exact(cuda, storage):
+    shape, n = (33, 9, 8), 33 * 9 * 8
+    f = _fields(n, 6)
+    got = []
+    for arith in ("exact", "fast"):
+        b = Box(*shape, 1.9, storage=storage, arith=arith, quadric_limiters=(np.inf, 0.01, np.inf))
+        b.init(*f)
+        b.step(5)
+        got.append(b.fields())
+    # five collisions of some 500 operations on moments of O(0.1), each rounded to 2^-53 or 2^-24
+    eps = 5 * 500 * 0.1 * 2.0 ** (-53 if storage == "f64" else -24)
+    for k in ("rho", "vx", "vy", "vz"):
+        assert np.abs(got[0][k] - got[1][k]).max() <= eps

@@ -36,7 +36,9 @@ struct K17Rates {
     // folded constants of the FMA form (k17_collide_fast)
     T omo;                      // 1 - omega
     T mc3h;                     // -3 (1 - omega / 2)
-    T hP, hM, cD;               // 1/2 (1 - OxyyPxzz) qP, 1/2 (1 - OxyyMxzz) qM, (1 - Oxyz) qD
+    T lP, lM, lD;               // the limiters, at most 2^100 (beside it |m| is rounded away: the limiter is off), which
+                                // keeps 1 / (|m| + l) normal and the product of seven of them in a double finite
+    T hP, hM, cD;               // 1/2 (1 - OxyyPxzz) lP, 1/2 (1 - OxyyMxzz) lM, (1 - Oxyz) lD
     T kA, kB;                   // neg_iwm 2/3 factorA, neg_iwm 1/3 factorB (-3 omega)
 };
 
@@ -65,9 +67,13 @@ inline K17Rates<T> make_k17_rates(T omega, T qP, T qM, T qD)
     r.omOM = T(1) - r.OxyyMxzz;
     r.omo = T(1) - w;
     r.mc3h = T(-3) * (T(1) - T(0.5) * w);
-    r.hP = T(0.5) * r.omOP * qP;
-    r.hM = T(0.5) * r.omOM * qM;
-    r.cD = r.omOxyz * qD;
+    const T most = T(0x1p100);
+    r.lP = qP > most ? most : qP;
+    r.lM = qM > most ? most : qM;
+    r.lD = qD > most ? most : qD;
+    r.hP = T(0.5) * r.omOP * r.lP;
+    r.hM = T(0.5) * r.omOM * r.lM;
+    r.cD = r.omOxyz * r.lD;
     r.kA = r.neg_iwm * (T(2) / T(3)) * r.factorA;
     r.kB = r.neg_iwm * (T(1) / T(3)) * r.factorB * r.m3w;
     return r;
@@ -713,7 +719,7 @@ __host__ __device__ __forceinline__ void k17_collide_fast(T *f, const K17Rates<B
 
     // third order with the quartic limiter (K17...h:397-433)
     const T lm[7] = { k111, k210 + k012, k201 + k021, k120 + k102, k210 - k012, k201 - k021, k120 - k102 };
-    const B lq[7] = { r.qD, r.qP, r.qP, r.qP, r.qM, r.qM, r.qM };
+    const B lq[7] = { r.lD, r.lP, r.lP, r.lP, r.lM, r.lM, r.lM };
     T li[7];
     limiter_inverses(lm, lq, li);
     const T c111 = (lm[0] * T(r.cD)) * li[0];

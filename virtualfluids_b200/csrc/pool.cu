@@ -33,6 +33,7 @@ int pool_cuda(cudaError_t e, const char *what)
         return VFB_OK;
     const std::string m = std::string(what) + ": " + cudaGetErrorString(e);
     vfb::set_last_error(m.c_str());
+    cudaGetLastError();                // reported by this call, not by the next one's launch
     return e == cudaErrorMemoryAllocation ? VFB_ERR_OUT_OF_MEMORY : VFB_ERR_CUDA;
 }
 
@@ -324,6 +325,10 @@ cudaError_t rebuild_list(vfb_pool *p, cudaStream_t s)
         drop_graph(p);                 // another kernel, with its own persistent grid
         p->narrow = narrow;
         e = update_grid(p);
+        if (e != cudaSuccess) {
+            p->narrow = !narrow;       // the grid is still the other kernel's
+            return e;
+        }
     }
     if (items.size() > p->items_capacity) {
         // a new buffer: a captured step refers to the old one
@@ -353,7 +358,7 @@ cudaError_t rebuild_list(vfb_pool *p, cudaStream_t s)
     if (e == cudaSuccess)
         reclaim(p);
     p->active_nodes = nodes;
-    p->list_dirty = false;
+    p->list_dirty = e != cudaSuccess;  // a list that did not arrive is formed again by the next call
     return e;
 }
 

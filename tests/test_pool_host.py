@@ -88,3 +88,15 @@ def test_a_work_list_without_memory_is_formed_again(lib):
     assert p.step() != 0 and lib.fake_launches() == before
     assert p.step() == 0 and p.last_launch() == (True, 9 * 64 ** 3 // (128 * 8), 128)
     p.close()
+
+
+@pytest.mark.parametrize("storage,width", [(N.STORAGE_F64, 1), (N.STORAGE_F32, 2), (N.STORAGE_F16, 2)], ids=["f64", "f32", "f16"])
+@pytest.mark.parametrize("nodes_per_thread", [1, 2, 3, 8])
+def test_items_hold_whole_multiples_of_a_threads_nodes(lib, storage, width, nodes_per_thread):
+    p = FakePool(lib, storage, 1)
+    p.set_launch(64, nodes_per_thread, -1)      # one block per item
+    p.add((40, 30, 20))
+    assert p.step() == 0
+    per_item = 64 * -(-nodes_per_thread // width) * width
+    assert p.last_launch()[1:] == (-(-24000 // per_item), 64)
+    p.close()

@@ -116,6 +116,7 @@ struct PoolDomainSpec {
                                         const uint32_t *n_items, int nodes_per_thread, bool even, bool narrow,     \
                                         unsigned grid, unsigned block, cudaStream_t s);                            \
         static const void *pool_kernel(bool even, bool narrow);                                                    \
+        static int pool_width(bool narrow);                                                                        \
         static size_t pool_domain_bytes();                                                                        \
         static void pool_domain(void *out, const PoolDomainSpec &spec);                                            \
         static cudaError_t pool_mass(void *arena, const void *domains, const uint2 *items, uint32_t n_items,       \

@@ -307,6 +307,13 @@ cudaError_t Launchers<S>::pool_collide(void *arena, const void *domains, const u
     return cudaGetLastError();
 }
 
+// nodes that a thread of the pool's collision takes at a time
+template <class S>
+int Launchers<S>::pool_width(bool narrow)
+{
+    return narrow && sizeof(S) <= 4 ? VFB_NS::pool_width<S, VFB_EXACT, true>() : VFB_NS::pool_width<S, VFB_EXACT, false>();
+}
+
 template <class S>
 const void *Launchers<S>::pool_kernel(bool even, bool narrow)
 {

@@ -155,9 +155,10 @@ class Pool:
         return [a.reshape(shape[2], shape[1], shape[0]) for a in out]
 
     def set_launch(self, threads=128, nodes_per_thread=8, blocks_per_sm=-1, use_graph=True):
-        """threads per block (64, 128, 256), nodes per thread per work item (1..32), resident blocks per
-        SM of the persistent launch (0: as many as fit; -1: one block per work item, no persistent
-        loop), CUDA-graph replay. Results do not depend on the shape."""
+        """threads per block (64, 128, 256), nodes per thread per work item (1..32; FMA arithmetic in FP32 takes two
+        at a time, so an odd number counts as the next even one), resident blocks per SM of the
+        persistent launch (0: as many as fit; -1: one block per work item, no persistent loop),
+        CUDA-graph replay. Results do not depend on the shape."""
         N.check(N.lib().vfb_pool_set_launch(self._h, int(threads), int(nodes_per_thread), int(blocks_per_sm),
                                             int(use_graph)))
 

@@ -454,8 +454,9 @@ int vfb_box_fields(vfb_box *box, void *rho, void *ux, void *uy, void *uz, int32_
 /* synchronises the stream and reads the status word the box's kernels set on a failed internal wait
    (0 = fine); returns VFB_ERR_CUDA when it is nonzero */
 int vfb_box_status(vfb_box *box, int32_t *device_status, void *stream);
-/* collision kernel: 0 = choose (two nodes per thread for FP32-arithmetic boxes of 151552 nodes and
-   more, else one), 1 = one node per thread, 2 = TMA-staged warp tiles (nx % 32 == 0),
+/* collision kernel: 0 = choose (two nodes per thread for FP32-arithmetic boxes of 200000 nodes and
+   more, with F16 or BF16 storage of 1600000 and more, else one), 1 = one node per thread,
+   2 = TMA-staged warp tiles (nx % 32 == 0),
    3 = per-thread asynchronous copies (F64 and F32 storage),
    4 = two nodes per thread in packed FP32x2 arithmetic (FP32 arithmetic; the bits of 1),
    5 = persistent blocks with the next node's loads in flight while the current node is collided */

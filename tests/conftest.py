@@ -1,3 +1,5 @@
+import ctypes
+import subprocess
 import sys
 from pathlib import Path
 
@@ -25,3 +27,18 @@ def cuda():
     if not torch.cuda.is_available():
         pytest.fail("a CUDA device is required for gpu-marked tests")
     return torch.device("cuda:0")
+
+
+@pytest.fixture(scope="session")
+def fake_lib(tmp_path_factory):
+    """The library on a CUDA runtime without a device (fake_cudart.cpp)."""
+    from virtualfluids_b200 import build as vbuild
+    vbuild.build()
+    out = tmp_path_factory.mktemp("fake") / "libvfb_fake.so"
+    # -Bsymbolic: the objects' calls go to the fake runtime whatever else the process has loaded
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I/usr/local/cuda/include",
+                    str(ROOT / "tests" / "fake_cudart.cpp"), *map(str, sorted(vbuild.BUILD.glob("*.o"))),
+                    "-Wl,-Bsymbolic", "-Wl,-z,defs", "-ldl", "-lrt", "-lpthread", "-o", str(out)], check=True)
+    lib = ctypes.CDLL(str(out))
+    lib.fake_launch.restype = ctypes.c_char_p
+    return lib

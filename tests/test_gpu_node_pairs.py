@@ -48,8 +48,10 @@ def test_two_nodes_per_thread_give_the_bits_of_one(cuda, storage, shape):
         assert np.allclose(one[2], two[2], rtol=1e-12, atol=0)
 
 
-@pytest.mark.parametrize("shape", [(53, 53, 53), (54, 53, 53)], ids=["below", "above"])
-def test_the_choice_by_size_changes_no_bit(cuda, shape):
-    assert shape == (53, 53, 53) or shape[0] * shape[1] * shape[2] >= 148 * 4 * 256
-    a, b = (_run(shape, "f32", v, 3) for v in ("auto", "direct"))
-    assert np.array_equal(a[0], b[0])
+# on either side of 200 000 (FP32, E3M12) and 1 600 000 nodes (FP16, BF16); tests/test_dispatch_host.py reads
+# which kernel a step launches there
+@pytest.mark.parametrize("storage,shape", [("f32", (57, 59, 59)), ("f32", (58, 59, 59)), ("e3m12", (58, 59, 59)),
+                                           ("f16", (116, 117, 117)), ("f16", (117, 117, 117)), ("bf16", (117, 117, 117))])
+def test_the_choice_by_size_changes_no_bit(cuda, storage, shape):
+    a, b, c = (_run(shape, storage, v, 3) for v in ("auto", "direct", "pairs"))
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[0], c[0])

@@ -2,30 +2,13 @@
 launches, on which grid, and what happens when a query fails. Domains of 4 GB a plane are address
 space only."""
 import ctypes as C
-import subprocess
-from pathlib import Path
 
 import pytest
 
 from virtualfluids_b200 import _native as N
-from virtualfluids_b200 import build as vbuild
 from virtualfluids_b200.pool import Pool
 
-ROOT = Path(__file__).resolve().parents[1]
 SMS, OCC_NARROW, OCC_WIDE = 148, 5, 3           # of the fake runtime
-
-
-@pytest.fixture(scope="module")
-def lib(tmp_path_factory):
-    vbuild.build()
-    out = tmp_path_factory.mktemp("fake") / "libvfb_fake.so"
-    # -Bsymbolic: the objects' calls go to the fake runtime whatever else the process has loaded
-    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I/usr/local/cuda/include",
-                    str(ROOT / "tests" / "fake_cudart.cpp"), *map(str, sorted(vbuild.BUILD.glob("*.o"))),
-                    "-Wl,-Bsymbolic", "-Wl,-z,defs", "-ldl", "-lrt", "-lpthread", "-o", str(out)], check=True)
-    so = C.CDLL(str(out))
-    so.fake_launch.restype = C.c_char_p
-    return so
 
 
 class FakePool:
@@ -62,38 +45,38 @@ class FakePool:
         self.lib.vfb_pool_destroy(self.h)
 
 
-def test_a_failed_change_of_kernel_is_reported_and_made_good(lib):
-    p = FakePool(lib, N.STORAGE_F32, 120)
+def test_a_failed_change_of_kernel_is_reported_and_made_good(fake_lib):
+    p = FakePool(fake_lib, N.STORAGE_F32, 120)
     p.set_launch(128, 8, 0)
     p.add((64, 64, 64))
     assert p.step() == 0 and p.last_launch() == (True, SMS * OCC_NARROW, 128)
     big = p.add((1024, 1024, 1024))             # planes of 4 GB: 64-bit slot offsets
-    lib.fake_fail_occupancy(1)
-    before = lib.fake_launches()
-    assert p.step() != 0 and lib.fake_launches() == before
+    fake_lib.fake_fail_occupancy(1)
+    before = fake_lib.fake_launches()
+    assert p.step() != 0 and fake_lib.fake_launches() == before
     assert p.step() == 0 and p.last_launch() == (False, SMS * OCC_WIDE, 128)
     p.remove(big)
     assert p.step() == 0 and p.last_launch() == (True, SMS * OCC_NARROW, 128)
     p.close()
 
 
-def test_a_work_list_without_memory_is_formed_again(lib):
-    p = FakePool(lib, N.STORAGE_F32, 1)
+def test_a_work_list_without_memory_is_formed_again(fake_lib):
+    p = FakePool(fake_lib, N.STORAGE_F32, 1)
     p.add((64, 64, 64))
     assert p.step() == 0
     for _ in range(8):
         p.add((64, 64, 64))                     # more items than the list holds
-    lib.fake_fail_malloc(1)
-    before = lib.fake_launches()
-    assert p.step() != 0 and lib.fake_launches() == before
+    fake_lib.fake_fail_malloc(1)
+    before = fake_lib.fake_launches()
+    assert p.step() != 0 and fake_lib.fake_launches() == before
     assert p.step() == 0 and p.last_launch() == (True, 9 * 64 ** 3 // (128 * 8), 128)
     p.close()
 
 
 @pytest.mark.parametrize("storage,width", [(N.STORAGE_F64, 1), (N.STORAGE_F32, 2), (N.STORAGE_F16, 2)], ids=["f64", "f32", "f16"])
 @pytest.mark.parametrize("nodes_per_thread", [1, 2, 3, 8])
-def test_items_hold_whole_multiples_of_a_threads_nodes(lib, storage, width, nodes_per_thread):
-    p = FakePool(lib, storage, 1)
+def test_items_hold_whole_multiples_of_a_threads_nodes(fake_lib, storage, width, nodes_per_thread):
+    p = FakePool(fake_lib, storage, 1)
     p.set_launch(64, nodes_per_thread, -1)      # one block per item
     p.add((40, 30, 20))
     assert p.step() == 0

@@ -98,7 +98,7 @@ class Box:
         return v.value
 
     def set_kernel_variant(self, variant: str):
-        """'auto' (two nodes per thread for FP32-arithmetic boxes that fill the device, else one),
+        """'auto' (two nodes per thread for large FP32-arithmetic boxes, else one),
         'direct' (one node per thread), 'tma' (bulk copies staged in shared memory), 'async'
         (per-thread asynchronous copies of the next node), 'pairs' (two nodes per thread in packed
         FP32x2 arithmetic; FP32-arithmetic forms) or 'pipe' (persistent blocks, the next node's loads

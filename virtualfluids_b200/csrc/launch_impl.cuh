@@ -103,8 +103,10 @@ cudaError_t Launchers<S>::k17_list(const vfb_level *L, const uint32_t *idx, uint
     const unsigned B = 128, G = grid1d(n, B);
     const bool even = L->is_even_timestep != 0;
     if constexpr (std::is_same<C, float>::value && !VFB_EXACT) {
-        // two entries per thread where they fill the device, as for a box (n < 2^31: 32-bit entry numbers)
-        if (slots && !wm && !bf && n >= 148u * 4u * 256u && n < (1u << 31)) {
+        // two entries per thread for large levels (32-bit entry numbers). Cavities, us per step with one and
+        // two: FP32 52^3 19.9 and 20.2, 54^3 21.2 and 15.6, 64^3 25.8 and 20.7, 96^3 71 and 66; replayed
+        // from a graph 54^3 15.1 and 15.6, 64^3 19.3 and 18.7, 96^3 64 and 59. FP16: the same lines
+        if (slots && !wm && !bf && n >= 151552u && n < (1u << 31)) {
             const unsigned G2 = grid1d(((uint64_t)n + 1) / 2, B);
             if (even) launch_next(k17_list_pair_kernel<S, true>, G2, B, s, a);
             else launch_next(k17_list_pair_kernel<S, false>, G2, B, s, a);
@@ -769,6 +771,16 @@ void launch_box_direct(const BoxCollideArgs<typename Codec<S>::compute> &a, bool
 }
 } // namespace
 
+// The nodes from which a box takes two per thread. us per step with one and two: FP32 52^3 5.9 and 6.3, 58^3
+// 8.0 and 8.2, 60^3 8.3 and 8.3, 64^3 9.6 and 8.9, 128^3 90 and 76; E3M12 50 to 58^3 within 3 %, 64^3 12.2
+// and 11.5, 128^3 94 and 82. FP16 and BF16 gain once their populations (54 B per node) leave L2: FP16
+// 64^3 10.1 and 10.2, 96^3 29.6 and 30.6, 116^3 51.4 and 52.1, 120^3 60.2 and 57.9, 128^3 79 and 71.
+template <class S>
+constexpr uint32_t pair_nodes()
+{
+    return std::is_same<S, __half>::value || std::is_same<S, __nv_bfloat16>::value ? 1600000u : 200000u;
+}
+
 template <class S>
 cudaError_t Launchers<S>::box_collide(const BoxState &b, bool even, double *partials, uint64_t *n_partials, cudaStream_t s)
 {
@@ -809,10 +821,7 @@ cudaError_t Launchers<S>::box_collide(const BoxState &b, bool even, double *part
 #undef VFB_K17Q
     }
     if constexpr (std::is_same<C, float>::value && !VFB_EXACT) {
-        // two nodes per thread where they fill the device: 148 SMs x 4 blocks x 256 nodes. Below
-        // that one node per thread spreads the box over more warps (32^3 in FP32: 4.1 against 6.2 us
-        // per step; 64^3: equal)
-        if (b.variant == 4 || (b.variant == 0 && a.count >= 148u * 4u * 256u)) {
+        if (b.variant == 4 || (b.variant == 0 && a.count >= pair_nodes<S>())) {
             const unsigned B = box_threads(a.count / 2), G = grid1d(((uint64_t)a.count + 1) / 2, B);
             if (n_partials)
                 *n_partials = (uint64_t)G * (B / 32);

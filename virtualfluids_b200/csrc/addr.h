@@ -11,8 +11,14 @@ struct NodeAddr {
     int nx, ny, nz, periodic;
 };
 
-// whether a direction plane of `nodes` nodes can be addressed with 32-bit byte offsets (slot_at)
-inline bool narrow_planes(uint64_t nodes, uint64_t storage_bytes) { return nodes * storage_bytes < (1ull << 32); }
+// whether a direction plane of `nodes` nodes is addressed with 32-bit byte offsets (PlaneNarrow): below
+// 4 GB; the bounds-checked build takes the 64-bit kernels from 1 MB, where small pools reach them
+#ifdef VFB_BOUNDS_CHECK
+constexpr uint64_t kNarrowBytes = 1ull << 20;
+#else
+constexpr uint64_t kNarrowBytes = 1ull << 32;
+#endif
+inline bool narrow_planes(uint64_t nodes, uint64_t storage_bytes) { return nodes * storage_bytes < kNarrowBytes; }
 
 // Division by a run-time constant d in [1, 2^16) of dividends n < 2^31 with one wide multiply and a
 // shift (Granlund and Montgomery, "Division by invariant integers using multiplication", PLDI

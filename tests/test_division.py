@@ -2,9 +2,11 @@
 
 refine_rcp and refine_div, the part without a branch: for every seed within 2^-18 of the reciprocal,
 with fractions at both ends of a binade (the all-ones divisor, where the last refinement alone gives
-the wrong neighbour; powers of two) and over wide exponents. rcp_rounded and div_rounded, the whole: for
-any operands (both signs, zeros, subnormals, infinities, NaN, exponents around the limits of the range that
-the first part serves), on the host and on the device with the hardware's approximation as seed."""
+the wrong neighbour; powers of two) and over wide exponents. rcp_rounded and limited, the whole: for any
+operands (both signs, zeros, subnormals, infinities, NaN, exponents around the limits of the range that the
+first part serves) and any limiters, on the host and on the device with the hardware's approximation. The
+collision's own 1 / rho has no branch: where rho is 0, infinite or huge, its populations must be those with
+the IEEE reciprocal all the same."""
 import ctypes
 import subprocess
 from pathlib import Path
@@ -36,6 +38,11 @@ def test_rounded_division_is_the_ieee_division(check, exponents):
 @pytest.mark.parametrize("wide", [0, 1], ids=["in_range", "any"])
 def test_whole_division_is_the_ieee_division(check, wide):
     assert check.whole_mismatches(300_000, wide) == 0
+
+
+def test_populations_where_the_density_has_no_reciprocal(check):
+    check.density_mismatches.argtypes, check.density_mismatches.restype = [ctypes.c_long], ctypes.c_long
+    assert check.density_mismatches(40_000) == 0
 
 
 @pytest.mark.gpu

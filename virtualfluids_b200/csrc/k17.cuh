@@ -33,6 +33,7 @@ struct K17Rates {
     T m3w;                      // -3 * omega
     T c3a;                      // 3 * (1 + 1/2 * (-omega))
     T omOxyz, omOP, omOM;       // 1 - Oxyz, 1 - OxyyPxzz, 1 - OxyyMxzz
+    T divBound;                 // the exact form's division without a branch (limited)
     // folded constants of the FMA form (k17_collide_fast)
     T omo;                      // 1 - omega
     T mc3h;                     // -3 (1 - omega / 2)
@@ -41,6 +42,20 @@ struct K17Rates {
     T hP, hM, cD;               // 1/2 (1 - OxyyPxzz) lP, 1/2 (1 - OxyyMxzz) lM, (1 - Oxyz) lD
     T kA, kB;                   // neg_iwm 2/3 factorA, neg_iwm 1/3 factorB (-3 omega)
 };
+
+namespace k17detail {
+// The bound of |m| + q below which limited() divides without a branch: 2^120 where the limiters q and the
+// rates O and o = 1 - O are ordinary, else 0.
+inline double division_bound(const double (&q)[3], const double (&O)[3], const double (&o)[3])
+{
+    bool fine = true;
+    for (int i = 0; i < 3; ++i)
+        fine = fine && q[i] >= 0x1p-300 && q[i] <= 0x1p100 && (o[i] == 0 || (std::fabs(o[i]) >= 0x1p-50 && std::fabs(o[i]) <= 0x1p50))
+            && (O[i] == 0 || std::fabs(O[i]) >= 0x1p-100);
+    return fine ? 0x1p120 : 0.0;
+}
+inline float division_bound(const float (&)[3], const float (&)[3], const float (&)[3]) { return 0.0f; }
+} // namespace k17detail
 
 // host computation of the omega-only rates, expression for expression as the reference
 template <class T>
@@ -65,6 +80,7 @@ inline K17Rates<T> make_k17_rates(T omega, T qP, T qM, T qD)
     r.omOxyz = T(1) - r.Oxyz;
     r.omOP = T(1) - r.OxyyPxzz;
     r.omOM = T(1) - r.OxyyMxzz;
+    r.divBound = k17detail::division_bound({ qP, qM, qD }, { r.OxyyPxzz, r.OxyyMxzz, r.Oxyz }, { r.omOP, r.omOM, r.omOxyz });
     r.omo = T(1) - w;
     r.mc3h = T(-3) * (T(1) - T(0.5) * w);
     const T most = T(0x1p100);
@@ -196,8 +212,8 @@ template <class T> __host__ __device__ __forceinline__ T k_y(int a, int c)
 //    the next double (its last bit set);
 //  * with y2 the rounded reciprocal, q1 = q0 - y2 (b q0 - a), one rounding, is the rounded quotient
 //    (the remainder is exact; in this sign a zero keeps that of the quotient).
-// The range is that of div_in_range for |b| and |a|, where a zero a wants a positive b: the quotient then
-// lies within 2^-960 and 2^960, and the remainder, a multiple of 2^-106 |a|, above the smallest double.
+// It holds for |b| in [2^-840, 2^120) and, with it, |a| in [2^-890, 2^170) or zero (b > 0 then): the
+// quotient is normal, and the remainder, a multiple of 2^-106 |a|, above the smallest double.
 __host__ __device__ __forceinline__ double refine_rcp(double b, double y)
 {
     const double e = ::fma(-b, y, 1.0);
@@ -222,8 +238,6 @@ __host__ __device__ __forceinline__ double refine_div(double a, double b, double
     return ::fma(-::fma(b, q, -a), y, q);
 }
 
-// x in [2^-840, 2^120), from its upper word
-__host__ __device__ __forceinline__ bool div_in_range(unsigned hi) { return hi - ((1023u - 840u) << 20) < (960u << 20); }
 __host__ __device__ __forceinline__ unsigned upper_word(double x)
 {
 #ifdef __CUDA_ARCH__
@@ -232,14 +246,6 @@ __host__ __device__ __forceinline__ unsigned upper_word(double x)
     uint64_t bits;
     __builtin_memcpy(&bits, &x, 8);
     return (unsigned)(bits >> 32);
-#endif
-}
-__host__ __device__ __forceinline__ bool is_zero(double x)
-{
-#ifdef __CUDA_ARCH__
-    return (((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x)) == 0u;
-#else
-    return x == 0.0;
 #endif
 }
 // an approximation of 1 / b: the hardware's, on the host one of 20 bits
@@ -259,39 +265,56 @@ __host__ __device__ __forceinline__ double rcp_seed(double b)
 #endif
 }
 
-// 1 / b and the quotients a[i] / b[i]. One branch for all of them leads to the compiler's divisions, for
-// operands out of range (infinite or NaN ones, a limiter of 1e40, a moment of 1e-260, a negative b[i]).
-// The compiler's division has such a branch in each of the eight, between which no arithmetic moves: four
-// exact FP64 steps of a 256^3 box took 6.90 ms with it and 6.63 ms with no branch at all; this branch
-// costs 0.09 ms of that.
+// 1 / b for any b
 __host__ __device__ __forceinline__ double rcp_rounded(double b)
 {
-    return div_in_range(upper_word(b) & 0x7fffffffu) ? refine_rcp(b, rcp_seed(b)) : 1.0 / b;
+    const bool fine = (upper_word(b) & 0x7fffffffu) - ((1023u - 840u) << 20) < (960u << 20);
+    return fine ? refine_rcp(b, rcp_seed(b)) : 1.0 / b;
 }
+__host__ __device__ __forceinline__ float rcp_rounded(float b) { return 1.0f / b; }
+// 1 / rho of the collision, without a branch (rho = 1 + drho is 0 or at least 2^-53 away from it). It is NaN
+// for a rho of 0 or infinity and 0 about 2^1022 and above; with the IEEE reciprocals there, too, all 27
+// populations come out NaN. The branch of rcp_rounded, on which all that follows waits, costs 1.6 % of the
+// exact collision: it is taken where the velocity is an output.
+__host__ __device__ __forceinline__ double rcp_density(double rho) { return refine_rcp(rho, rcp_seed(rho)); }
+__host__ __device__ __forceinline__ float rcp_density(float rho) { return 1.0f / rho; }
+
+// The third order moments m, limited: m + (O + o |m| / (|m| + q)) (-m), the IEEE quotients. One test for
+// all of them sends any operand out of the range of refine_div to the compiler's division: |m| + q at
+// the bound, infinite or NaN, or 0 < |m| < 2^-840 (a limiter of 1e40, a moment of 1e-260). An |m| below
+// 2^-1042 counts as zero in it, which changes nothing: its quotient, below 2^-690, vanishes beside O,
+// or, where O is 0, beside 1 in m's own product.
+// The compiler's division has such a branch in each of the seven, between which no arithmetic moves: four
+// exact FP64 steps of 256^3 took 6.90 ms with it and 6.63 ms with no branch at all. This one costs 0.8 %.
 template <int N>
-__host__ __device__ __forceinline__ void div_rounded(const double (&a)[N], const double (&b)[N], double (&q)[N])
+__host__ __device__ __forceinline__ void limited(double (&m)[N], const double (&O)[N], const double (&o)[N],
+                                                 const double (&q)[N], double bound)
 {
     bool fine = true;
+    double w[N];
 #pragma unroll
     for (int i = 0; i < N; ++i)
-        fine &= div_in_range(upper_word(b[i])) & (div_in_range(upper_word(a[i]) & 0x7fffffffu) | is_zero(a[i]));
+        fine &= (upper_word(fabs(m[i]) + q[i]) < upper_word(bound)) & (2u * upper_word(m[i]) - 2u >= 2u * ((1023u - 840u) << 20) - 2u);
     if (fine) {
 #pragma unroll
         for (int i = 0; i < N; ++i)
-            q[i] = refine_div(a[i], b[i], rcp_seed(b[i]));
+            w[i] = refine_div(o[i] * fabs(m[i]), fabs(m[i]) + q[i], rcp_seed(fabs(m[i]) + q[i]));
     } else {
 #pragma unroll
         for (int i = 0; i < N; ++i)
-            q[i] = a[i] / b[i];
+            w[i] = o[i] * fabs(m[i]) / (fabs(m[i]) + q[i]);
     }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        m[i] += (O[i] + w[i]) * (-m[i]);
 }
-__host__ __device__ __forceinline__ float rcp_rounded(float b) { return 1.0f / b; }
 template <int N>
-__host__ __device__ __forceinline__ void div_rounded(const float (&a)[N], const float (&b)[N], float (&q)[N])
+__host__ __device__ __forceinline__ void limited(float (&m)[N], const float (&O)[N], const float (&o)[N],
+                                                 const float (&q)[N], float)
 {
 #pragma unroll
     for (int i = 0; i < N; ++i)
-        q[i] = a[i] / b[i];
+        m[i] += (O[i] + o[i] * fabsf(m[i]) / (fabsf(m[i]) + q[i])) * (-m[i]);
 }
 
 } // namespace k17detail
@@ -328,14 +351,14 @@ __host__ __device__ __forceinline__ T momentum_z(const T *f)
 }
 
 // In place on f[27] (direction order). fx, fy, fz: half the acceleration, already scaled.
-// Returns drho and the velocity including the half force (MacroscopicValues).
-template <class T, bool EXACT>
+// Returns drho and the velocity including the half force (MacroscopicValues); VELOCITY: the caller keeps it.
+template <class T, bool EXACT, bool VELOCITY = false>
 __host__ __device__ __forceinline__ void k17_collide(T *f, const K17Rates<T> &r, T fx, T fy, T fz, T &drho_out, T &vx_out,
                                             T &vy_out, T &vz_out)
 {
     using namespace k17detail;
     const T drho = density_pyramid(f);
-    const T oneOverRho = rcp_rounded(drho + T(1));
+    const T oneOverRho = VELOCITY ? rcp_rounded(drho + T(1)) : rcp_density(drho + T(1));
     T vx = momentum_x(f) * oneOverRho;
     T vy = momentum_y(f) * oneOverRho;
     T vz = momentum_z(f) * oneOverRho;
@@ -411,21 +434,18 @@ __host__ __device__ __forceinline__ void k17_collide(T *f, const K17Rates<T> &r,
     M(1, 1, 0) += omega * (-M(1, 1, 0));
 
     // third order with the quartic limiter (K17...h:397-410)
-    const T size[7] = { fabs(M(1, 1, 1)), fabs(mxxyPyzz), fabs(mxxyMyzz), fabs(mxxzPyyz), fabs(mxxzMyyz), fabs(mxyyPxzz),
-                        fabs(mxyyMxzz) };
-    const T above[7] = { r.omOxyz * size[0], r.omOP * size[1], r.omOM * size[2], r.omOP * size[3], r.omOM * size[4],
-                         r.omOP * size[5], r.omOM * size[6] };
-    const T below[7] = { size[0] + r.qD, size[1] + r.qP, size[2] + r.qM, size[3] + r.qP, size[4] + r.qM, size[5] + r.qP,
-                         size[6] + r.qM };
-    T lim[7];
-    div_rounded(above, below, lim);
-    M(1, 1, 1) += (r.Oxyz + lim[0]) * (-M(1, 1, 1));
-    mxxyPyzz += (r.OxyyPxzz + lim[1]) * (-mxxyPyzz);
-    mxxyMyzz += (r.OxyyMxzz + lim[2]) * (-mxxyMyzz);
-    mxxzPyyz += (r.OxyyPxzz + lim[3]) * (-mxxzPyyz);
-    mxxzMyyz += (r.OxyyMxzz + lim[4]) * (-mxxzMyyz);
-    mxyyPxzz += (r.OxyyPxzz + lim[5]) * (-mxyyPxzz);
-    mxyyMxzz += (r.OxyyMxzz + lim[6]) * (-mxyyMxzz);
+    T third[7] = { M(1, 1, 1), mxxyPyzz, mxxyMyzz, mxxzPyyz, mxxzMyyz, mxyyPxzz, mxyyMxzz };
+    const T O[7] = { r.Oxyz, r.OxyyPxzz, r.OxyyMxzz, r.OxyyPxzz, r.OxyyMxzz, r.OxyyPxzz, r.OxyyMxzz };
+    const T o[7] = { r.omOxyz, r.omOP, r.omOM, r.omOP, r.omOM, r.omOP, r.omOM };
+    const T q[7] = { r.qD, r.qP, r.qM, r.qP, r.qM, r.qP, r.qM };
+    limited(third, O, o, q, r.divBound);
+    M(1, 1, 1) = third[0];
+    mxxyPyzz = third[1];
+    mxxyMyzz = third[2];
+    mxxzPyyz = third[3];
+    mxxzMyyz = third[4];
+    mxyyPxzz = third[5];
+    mxyyMxzz = third[6];
 
     // back from the linear combinations (K17...h:424-433)
     M(2, 0, 0) = c13 * (mxxMyy + mxxMzz + mxxPyyPzz);
@@ -819,11 +839,11 @@ __host__ __device__ __forceinline__ void k17_collide_fast(T *f, const K17Rates<B
 
 namespace vfb {
 // the collision of the chosen arithmetic variant
-template <class T, bool EXACT>
+template <class T, bool EXACT, bool VELOCITY = false>
 __host__ __device__ __forceinline__ void collide(T *f, const K17Rates<T> &r, T fx, T fy, T fz, T &drho, T &vx, T &vy, T &vz)
 {
     if constexpr (EXACT) {
-        k17_collide<T, true>(f, r, fx, fy, fz, drho, vx, vy, vz);
+        k17_collide<T, true, VELOCITY>(f, r, fx, fy, fz, drho, vx, vy, vz);
     } else {
         Rn<T> g[27], out[4];
 #pragma unroll

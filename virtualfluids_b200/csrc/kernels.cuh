@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(128) k17_list_kernel(ListCollideArgs<typename 
     C f[27];
     gather_planes<S, EVEN>(planes_of<S, EXACT>(a.planes, a.n), nodes, f);
     C drho, vx, vy, vz;
-    collide<C, EXACT>(f, a.rates, fx, fy, fz, drho, vx, vy, vz);
+    collide<C, EXACT, WRITE_MACRO>(f, a.rates, fx, fy, fz, drho, vx, vy, vz);
     if (WRITE_MACRO) {
         a.vx[k] = vx;
         a.vy[k] = vy;

@@ -994,8 +994,8 @@ static int detect_regular_box(SimLevel &S)
     S.regular = false;
     const vfb_level &L = S.level;
     const uint32_t n = S.n_fluid;
-    // the 16-bit forms hash each slot's offset into their stochastic rounding: a box over the
-    // shifted array would round differently, so they keep the list kernel
+    // the 16-bit forms hash each slot's node number into their stochastic rounding: a box, which
+    // numbers the same nodes from 0, would round differently, so they keep the list kernel
     if (L.storage != VFB_STORAGE_F64 && L.storage != VFB_STORAGE_F32)
         return VFB_OK;
     if (n < 2 || !L.neighbor_x || !L.neighbor_y || !L.neighbor_z)
@@ -1062,7 +1062,7 @@ static double list_half_force(const vfb_level &L, int axis)
 }
 
 // a regular level as a structured box over the reference layout: the populations of node
-// box_first + k at plane * numberOfNodes + box_first + k, the direct-load box kernel
+// box_first + k at plane * numberOfNodes + box_first + k, with one or two nodes per thread by its size
 static vfb::BoxState regular_box_state(const SimLevel &S)
 {
     const vfb_level &L = S.level;

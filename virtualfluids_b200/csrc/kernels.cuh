@@ -48,8 +48,9 @@ __device__ __forceinline__ uint32_t checked_node(uint32_t v, uint64_t n)
 
 // Where the 27 direction planes start. In the kernels' parameters (PlaneTable) a plane's pointer is a
 // constant operand of the one multiply-add that forms a slot's address; formed from a base and a
-// stride, every slot costs two additions more (FP16, two nodes per thread: 1576 against 1456
-// instructions, FP32 1320 against 1184, and registers to spare). PlaneStride serves the kernels
+// stride, every slot costs two additions more (warp instructions per two nodes on 176^3, table against
+// stride: FP32 1057 and 1228, FP16 1344 and 1491, E3M12 1767 and 1915; FP32 320 x 256 x 192 531 and 618 us
+// per step, E3M12 256^3 628 and 657, FP16 250 x 190 x 230 362 and 365). PlaneStride serves the kernels
 // that are bound by something else.
 struct PlaneTable {
     void *p[27];
@@ -229,9 +230,9 @@ __device__ __forceinline__ void node_slots(uint32_t k, const uint32_t *nbx, cons
         box_nodes(k, b, nodes);
 }
 
-// Which one-node kernels take the table: the exact FP64 ones (0.8 %). FP64 with FMA arithmetic was 6 %
-// slower with it (256^3 1205 against 1130 us per step), the FP32-arithmetic forms no faster, and a
-// small box lost 4 % to reading 27 pointers per launch (64 steps of 32^3 228 against 220 us).
+// Which one-node kernels take the table: the exact FP64 ones (256^3 1338 against 1377 us per step, 96^3 75.1
+// against 77.5). FP64 with FMA arithmetic is slower with it (256^3 1206 against 1130 us), the FP32-arithmetic
+// forms no faster (FP32 320 x 256 x 192 664 against 662, FP16 250 x 190 x 230 406 against 403).
 template <class S, bool EXACT>
 constexpr bool plane_table_pays() { return sizeof(S) == 8 && EXACT; }
 template <class S, bool EXACT>
@@ -323,7 +324,7 @@ __device__ __forceinline__ void collide_two(const P &planes, const uint32_t (&na
         f[d] = f2(fa[d], fb[d]);
     k17_collide_fast<f2, float>(f, r, fx, fy, fz, m[0], m[1], m[2], m[3]);
     // the encoding products in one instruction for both nodes; E3M12's results are subnormal floats,
-    // with which the packed product is slower than two scalar ones (778 against 671 us on 256^3)
+    // with which the packed product is slower than two scalar ones (256^3 640 against 628 us)
 #pragma unroll
     for (int d = 0; d < 27; ++d) {
         if constexpr (Codec<S>::kPackedScale)
@@ -521,8 +522,8 @@ __global__ void __launch_bounds__(128) k17_list_staged_kernel(ListCollideArgs<ty
 // each row left part of the last block of a row without nodes but not without registers.
 // ---------------------------------------------------------------------------------------------
 // resident blocks per SM the register budget must allow: three for FP64 arithmetic (at most 168
-// registers; an unbounded build of the exact energy variant takes 170, which rounds to 176 and
-// leaves two), four for FP32 arithmetic (at most 128)
+// registers), four for FP32 arithmetic (at most 128). The exact FP64 kernel would fit four as well (126
+// registers): 256^3 1.267 against 1.310 ms per step, but 24^3 7.4 against 4.8 us, 36^3 8.1 against 6.7
 template <class S>
 constexpr int box_min_blocks() { return sizeof(typename Codec<S>::compute) == 8 ? 3 : 4; }
 
@@ -756,9 +757,10 @@ __global__ void __launch_bounds__(128, pipe_min_blocks<S>()) k17_box_pipe_kernel
 // (a warp owns 64 consecutive nodes), collided together in packed FP32x2 arithmetic (packed.cuh):
 // the arithmetic issues half the instructions, every access stays a full warp's in order, and
 // each node's bits are those of k17_box_kernel. FMA arithmetic only. Bound: HBM and its latency
-// (FP32), issue and the FMA pipe (16-bit forms). Four blocks per SM (128 registers, no more than a
-// few spilled) beat three (150 registers): FP32 320 x 256 x 192 589 against 621 us per step, where
-// one node per thread takes 661; FP16 250 x 190 x 230 369 us against 412 with one node.
+// (FP32), issue and the FMA pipe (16-bit forms). Now, with two nodes against one: FP32 320 x 256 x 192
+// 531 against 662 us per step, FP16 250 x 190 x 230 362 against 403. Four blocks per SM (128
+// registers, no more than a few spilled) beat three (150 registers): before the planes' pointers came
+// as parameters FP32 589 against 621 us.
 // ---------------------------------------------------------------------------------------------
 template <class S, bool EVEN, bool MASK, bool ENERGY>
 __global__ void __launch_bounds__(128, 4) k17_box_pair_kernel(BoxCollideArgs<float> a)

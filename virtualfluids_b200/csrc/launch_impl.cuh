@@ -17,9 +17,9 @@ namespace VFB_NS {
 
 namespace {
 // A kernel that begins with chain_begin, placed on the device while the kernel before it in the
-// stream still runs (errors are read by cudaGetLastError as for any launch). 64 steps of a 32^3 FP32
-// box with set-up and output 275 -> 224 us, the 64^3 cavity's 20 steps 1024 -> 890 us. Not inside a
-// capture: replayed as programmatic edges the same kernels are slower than with full ones (32
+// stream still runs (errors are read by cudaGetLastError as for any launch). A step of a 32^3 FP32 box
+// 5.2 -> 3.8 us, 20 steps of the 64^3 cavity 1040 -> 849 us, 10 of a refined box 496 -> 408 us. Not inside a
+// capture: replayed as programmatic edges the same kernels were slower than with full ones (32
 // steps of a channel 2490 against 2270 us, of porous blocks 7420 against 6940 us).
 template <class... P, class... A>
 inline void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, const A &...args)

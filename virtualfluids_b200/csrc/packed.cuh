@@ -28,9 +28,9 @@ __host__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.
 __host__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 __host__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
 #endif
-// a - b = b * (-1) + a: the product is exact, so one rounding as in the scalar subtraction
 __host__ __device__ __forceinline__ f2 wrap(float2 v) { f2 r; r.v = v; return r; }
 __host__ __device__ __forceinline__ f2 operator+(f2 a, f2 b) { return wrap(add2(a.v, b.v)); }
+// a - b = b * (-1) + a: the product is exact, so one rounding as in the scalar subtraction
 __host__ __device__ __forceinline__ f2 operator-(f2 a, f2 b) { return wrap(fma2(b.v, make_float2(-1.0f, -1.0f), a.v)); }
 __host__ __device__ __forceinline__ f2 operator*(f2 a, f2 b) { return wrap(mul2(a.v, b.v)); }
 __host__ __device__ __forceinline__ f2 operator-(f2 a) { return f2(-a.v.x, -a.v.y); }

@@ -49,7 +49,7 @@ U0 = 0.04
 RE = 1600.0
 BYTES_PER_NODE = {"f64": 432, "f32": 216, "f16": 108, "bf16": 108, "e3m12": 108}
 # DRAM bytes (read + write) per node of one launch of the FP64 one-node collision kernel of each
-# arithmetic, from one ncu capture each at 128^3 (2,097,152 nodes; profiles/k17_box_kernel_f64_*);
+# arithmetic, from one ncu capture each at 128^3 (2,097,152 nodes);
 # traffic grows with the node count, so it is scaled to the bench's box
 NCU_DRAM_BYTES_PER_NODE_F64 = {"fast": (453.008384e6 + 396.124416e6) / 2097152,
                                "exact": (453.020160e6 + 394.798592e6) / 2097152}

@@ -141,7 +141,7 @@ extern "C" long whole_mismatches(long cases, int wide)
 }
 extern "C" long density_mismatches(long cases)
 {
-    const auto r = vfb::make_k17_rates<double>(1.9, 0.01, 0.01, 0.01);
+    const auto r = vfb::make_k17_rates<double>(1.9, 0.01, 0.01, 0.01, true);
     long bad = 0;
     for (long i = 0; i < cases; ++i) {
         double f[2][27], out[2][4];

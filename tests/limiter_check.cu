@@ -9,7 +9,8 @@
 template <class T>
 static double largest_difference(double qP, double qM, double qD, int cases)
 {
-    const auto r = vfb::make_k17_rates<T>(T(1.9), T(qP), T(qM), T(qD));
+    const auto exact = vfb::make_k17_rates<T>(T(1.9), T(qP), T(qM), T(qD), true);
+    const auto fma = vfb::make_k17_rates<T>(T(1.9), T(qP), T(qM), T(qD), false);
     uint64_t h = 0x9E3779B97F4A7C15ull;
     double worst = 0;
     for (int i = 0; i < cases; ++i) {
@@ -20,8 +21,8 @@ static double largest_difference(double qP, double qM, double qD, int cases)
             h ^= h << 17;
             f[d] = g[d] = T((double)(int64_t)h * 0x1p-63 * 0.02);
         }
-        vfb::collide<T, true>(f, r, T(0), T(0), T(0), m[0], m[1], m[2], m[3]);
-        vfb::collide<T, false>(g, r, T(0), T(0), T(0), m[0], m[1], m[2], m[3]);
+        vfb::collide<T, true>(f, exact, T(0), T(0), T(0), m[0], m[1], m[2], m[3]);
+        vfb::collide<T, false>(g, fma, T(0), T(0), T(0), m[0], m[1], m[2], m[3]);
         for (int d = 0; d < 27; ++d) {
             const double off = std::fabs((double)f[d] - (double)g[d]);
             if (!std::isfinite(off))

@@ -293,7 +293,7 @@ int vfb_k17_rates(double omega, double rates[6])
 {
     if (!rates)
         return fail(VFB_ERR_INVALID_ARGUMENT, "NULL rates");
-    const vfb::K17Rates<double> r = vfb::make_k17_rates<double>(omega, 0.01, 0.01, 0.01);
+    const vfb::K17Rates<double> r = vfb::make_k17_rates<double>(omega, 0.01, 0.01, 0.01, true);
     rates[0] = r.OxyyPxzz;
     rates[1] = r.OxyyMxzz;
     rates[2] = r.Oxyz;

@@ -26,21 +26,19 @@ struct K17Rates {
     T OxyyPxzz, OxyyMxzz, Oxyz; // 3rd order rates (K17...h:251-255)
     T factorA, factorB;         // 4th order diffusion parameters (K17...h:272-273)
     T neg_iwm;                  // -(1/omega - 1/2)
-    T qP, qM, qD;               // quadric limiters (Parameter.cpp:69 default 0.01)
+    T qP, qM, qD;               // quadric limiters (Parameter.cpp:69 default 0.01); FMA form: at most 2^100
     // omega-only subexpressions of the collision, each rounded as the reference rounds it in place
     T mhw;                      // 1/2 * (-omega) (exact)
     T w32;                      // omega * 3/2
     T m3w;                      // -3 * omega
     T c3a;                      // 3 * (1 + 1/2 * (-omega))
     T omOxyz, omOP, omOM;       // 1 - Oxyz, 1 - OxyyPxzz, 1 - OxyyMxzz
-    T divBound;                 // the exact form's division without a branch (limited)
     // folded constants of the FMA form (k17_collide_fast)
     T omo;                      // 1 - omega
     T mc3h;                     // -3 (1 - omega / 2)
-    T lP, lM, lD;               // the limiters, at most 2^100 (beside it |m| is rounded away: the limiter is off), which
-                                // keeps 1 / (|m| + l) normal and the product of seven of them in a double finite
-    T hP, hM, cD;               // 1/2 (1 - OxyyPxzz) lP, 1/2 (1 - OxyyMxzz) lM, (1 - Oxyz) lD
+    T hP, hM, cD;               // 1/2 (1 - OxyyPxzz) qP, 1/2 (1 - OxyyMxzz) qM, (1 - Oxyz) qD
     T kA, kB;                   // neg_iwm 2/3 factorA, neg_iwm 1/3 factorB (-3 omega)
+    T divBound;                 // the exact form's division without a branch (limited)
 };
 
 namespace k17detail {
@@ -57,10 +55,18 @@ inline double division_bound(const double (&q)[3], const double (&O)[3], const d
 inline float division_bound(const float (&)[3], const float (&)[3], const float (&)[3]) { return 0.0f; }
 } // namespace k17detail
 
-// host computation of the omega-only rates, expression for expression as the reference
+// host computation of the omega-only rates, expression for expression as the reference. The FMA form takes
+// limiters of at most 2^100: beside that |m| is rounded away (the limiter is off), and 1 / (|m| + q) stays
+// normal and the product of seven denominators in a double finite.
 template <class T>
-inline K17Rates<T> make_k17_rates(T omega, T qP, T qM, T qD)
+inline K17Rates<T> make_k17_rates(T omega, T qP, T qM, T qD, bool exact)
 {
+    const T most = T(0x1p100);
+    if (!exact) {
+        qP = qP > most ? most : qP;
+        qM = qM > most ? most : qM;
+        qD = qD > most ? most : qD;
+    }
     K17Rates<T> r;
     const T w = omega;
     r.omega = w;
@@ -83,13 +89,9 @@ inline K17Rates<T> make_k17_rates(T omega, T qP, T qM, T qD)
     r.divBound = k17detail::division_bound({ qP, qM, qD }, { r.OxyyPxzz, r.OxyyMxzz, r.Oxyz }, { r.omOP, r.omOM, r.omOxyz });
     r.omo = T(1) - w;
     r.mc3h = T(-3) * (T(1) - T(0.5) * w);
-    const T most = T(0x1p100);
-    r.lP = qP > most ? most : qP;
-    r.lM = qM > most ? most : qM;
-    r.lD = qD > most ? most : qD;
-    r.hP = T(0.5) * r.omOP * r.lP;
-    r.hM = T(0.5) * r.omOM * r.lM;
-    r.cD = r.omOxyz * r.lD;
+    r.hP = T(0.5) * r.omOP * qP;
+    r.hM = T(0.5) * r.omOM * qM;
+    r.cD = r.omOxyz * qD;
     r.kA = r.neg_iwm * (T(2) / T(3)) * r.factorA;
     r.kB = r.neg_iwm * (T(1) / T(3)) * r.factorB * r.m3w;
     return r;
@@ -739,7 +741,7 @@ __host__ __device__ __forceinline__ void k17_collide_fast(T *f, const K17Rates<B
 
     // third order with the quartic limiter (K17...h:397-433)
     const T lm[7] = { k111, k210 + k012, k201 + k021, k120 + k102, k210 - k012, k201 - k021, k120 - k102 };
-    const B lq[7] = { r.lD, r.lP, r.lP, r.lP, r.lM, r.lM, r.lM };
+    const B lq[7] = { r.qD, r.qP, r.qP, r.qP, r.qM, r.qM, r.qM };
     T li[7];
     limiter_inverses(lm, lq, li);
     const T c111 = (lm[0] * T(r.cD)) * li[0];

@@ -51,7 +51,7 @@ inline unsigned grid1d(uint64_t n, unsigned block) { return (unsigned)((n + bloc
 template <class C>
 K17Rates<C> rates_of(double omega, const double lim[3])
 {
-    return make_k17_rates<C>((C)omega, (C)lim[0], (C)lim[1], (C)lim[2]);
+    return make_k17_rates<C>((C)omega, (C)lim[0], (C)lim[1], (C)lim[2], VFB_EXACT);
 }
 
 // RunCollision.cuh:112-114: forces * c1o2 * forceFactor, forceFactor = 1/2^level (KernelUtilities.h:56)
